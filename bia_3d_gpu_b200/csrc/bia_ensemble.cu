@@ -21,6 +21,7 @@
 #include "bia_learned_block.cuh"
 #include "bia_pair.cuh"
 #include "bia_tiles.cuh"
+#include "bia_uv_walk.cuh"
 
 struct bia_ensemble {
     int nsys = 0;
@@ -67,8 +68,7 @@ struct EnsArgs {
 };
 
 // Each warp takes items t = (its global warp index) + k * (warps in the grid), as
-// bia_pair_tiles_kernel (a persistent grid for the universal-variable method, the counters
-// flushed per warp every kFlushBlocks items).
+// bia_pair_tiles_kernel (ALG and RKF45), the counters flushed per warp every kFlushBlocks items.
 template <int M>
 __global__ void __launch_bounds__(kEnsThreads, TileOccupancy<M>::kMinBlocks) ens_pair_tiles_kernel(const EnsArgs A)
 {
@@ -164,45 +164,40 @@ static int ens_phase_setup()
     return sms_of[dev];
 }
 
-// Learned step over the item table, first kernel: each item's pairs except the deferred ones
-// (rest_block_solve, rest_block_defer, as bia_pair_rest_kernel), the items holding deferred
-// pairs listed with their rows; the head kernel of the single-system step then evaluates the
-// rows and ens_pair_learned_finish_kernel solves the listed items' deferred pairs.
-__global__ void __launch_bounds__(kEnsThreads, 2) ens_pair_rest_kernel(const EnsArgs A)
-{
-    extern __shared__ __align__(16) uint8_t ens_rest_smem[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    double *ws = reinterpret_cast<double *>(ens_rest_smem + warp * kRestWarpBytes);
-    uint32_t *wslots = reinterpret_cast<uint32_t *>(ens_rest_smem + warp * kRestWarpBytes +
-                                                    kTileSmemDoubles * sizeof(double));
-    PairCounters tot;
-    counters_zero(tot);
-    int nblk = 0;
-    for (long long t = (long long)blockIdx.x * kEnsWarps + warp; t < A.nitems;
-         t += (long long)gridDim.x * kEnsWarps) {  // warp-uniform
+// The item table for uv_walk_blocks.
+struct EnsItems {
+    const EnsArgs &A;
+    __device__ __forceinline__ WalkBlock block(long long t) const
+    {
         const uint2 it = A.items[t];
-        const int s = (int)it.x;
-        const int bi = (int)(it.y & 0xffffu), bj = (int)(it.y >> 16);
+        WalkBlock B;
+        B.bi = (int)(it.y & 0xffffu);
+        B.bj = (int)(it.y >> 16);
+        B.sys = (int)it.x;
+        B.item = (unsigned int)t;
+        return B;
+    }
+    __device__ __forceinline__ WalkSystem system(int s) const
+    {
         const int base = A.off[s];
         const int n = A.off[s + 1] - base;
-        double racc[6], cacc[6];
-        uint32_t mask[kMlpHeads];
-        PairCounters cnt;
-        rest_block_solve(A.x + base, A.y + base, A.z + base, A.u + base, A.v + base, A.w + base,
-                         A.q ? A.q + base : nullptr, n, A.eps[s], A.P.dt, bi, bj, lane, ws, wslots, racc, cacc,
-                         mask, cnt);
-        counters_add(tot, cnt);
-        if (++nblk == kFlushBlocks) {
-            flush_counters(tot, A.stats, lane);
-            counters_zero(tot);
-            nblk = 0;
-        }
-        const int nb = (n + 31) / 32;
-        write_partials(A.part + A.part_off[s], (size_t)nb * 32, bi, bj, lane, racc, cacc);
-        rest_block_defer(A.R, (unsigned int)t, mask, wslots, lane);
+        return {A.x + base, A.y + base, A.z + base, A.u + base, A.v + base, A.w + base, A.q ? A.q + base : nullptr,
+                n, A.eps[s], A.part + A.part_off[s], (size_t)((n + 31) / 32) * 32};
     }
-    if (nblk > 0) flush_counters(tot, A.stats, lane);
+};
+
+// The universal-variable step (kRest false) and the learned step's first kernel over the item
+// table, as bia_pair_walk_kernel: the head kernel of the single-system step then evaluates the
+// deferred pairs' rows and ens_pair_learned_finish_kernel solves them.
+template <bool kRest>
+__global__ void __launch_bounds__(kEnsThreads, 2) ens_pair_walk_kernel(const EnsArgs A)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    WalkCounts c = {0, 0, 0, 0};
+    uv_walk_blocks<true, kRest>(EnsItems{A}, (long long)blockIdx.x * kEnsWarps + warp,
+                                (long long)gridDim.x * kEnsWarps, A.nitems, A.P.dt, warp * walk_warp_doubles<kRest>(),
+                                A.R, c);
+    walk_flush_counts(c, A.stats, lane);
 }
 
 // Learned step over the item table, third kernel (persistent 8-warp CTAs): a dense or
@@ -305,8 +300,8 @@ static int ens_learned_setup()
     const int hgrid = learned_head_grid();
     std::lock_guard<std::mutex> lk(mu);
     if (!done_of[dev]) {
-        ok_of[dev] = cudaFuncSetAttribute(ens_pair_rest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)kRestSmemBytes) == cudaSuccess;
+        ok_of[dev] = cudaFuncSetAttribute(ens_pair_walk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)walk_smem_bytes<true>(kEnsWarps)) == cudaSuccess;
         if (!ok_of[dev]) cudaGetLastError();
         done_of[dev] = true;
     }
@@ -445,7 +440,7 @@ static int ens_pair_launch(bia_context *ctx, bia_ensemble *E, EnsArgs &A, int me
         cudaError_t e = cudaMemsetAsync(A.R.counts, 0, kSplitHeader, st);
         if (e != cudaSuccess) return cuda_status(e);
         const unsigned rgrid = (unsigned)persistent_grid(grid);
-        ens_pair_rest_kernel<<<rgrid, kEnsThreads, kRestSmemBytes, st>>>(A);
+        ens_pair_walk_kernel<true><<<rgrid, kEnsThreads, walk_smem_bytes<true>(kEnsWarps), st>>>(A);
         long long hcap = lsetup;
         if (shape == 0 || shape == 1) hcap = (long long)device_sm_count() * (shape + 1);
         launch_learned_head(A.R, A.heads, A.stats, (int)hcap, st);
@@ -453,10 +448,10 @@ static int ens_pair_launch(bia_context *ctx, bia_ensemble *E, EnsArgs &A, int me
         return cuda_status(cudaGetLastError());
     }
     switch (method) {
-    case BIA_METHOD_RKF: ens_pair_tiles_kernel<kMethodRkf><<<grid, kEnsThreads, 0, st>>>(A); break;
+    case BIA_METHOD_RKF: ens_pair_tiles_kernel<kMethodRkf><<<grid, kEnsThreads, kSliceBytes, st>>>(A); break;
     case BIA_METHOD_UNIVERSAL:
-        ens_pair_tiles_kernel<kMethodUniversal>
-            <<<shape == 0 ? grid : (unsigned)persistent_grid(grid), kEnsThreads, 0, st>>>(A);
+        ens_pair_walk_kernel<false><<<shape == 0 ? grid : (unsigned)persistent_grid(grid), kEnsThreads,
+                                      walk_smem_bytes<false>(kEnsWarps), st>>>(A);
         break;
     default: {
         const int sms = BIA_PHASE_WARPS > 0 ? ens_phase_setup() : 0;

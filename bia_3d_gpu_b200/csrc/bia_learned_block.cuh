@@ -67,14 +67,13 @@ __device__ __forceinline__ void cta_scan2(MlpSmem &S, int a, int b, int &oa, int
 
 
 // The split learned step in three kernels, shared by the single-system step and the ensemble:
-//  rest    every pair gets the universal-variable prepare and the fifth-order start; a pair
-//          whose start is exact is composed right there.  A pair whose start is not exact and
-//          that lies inside a head's domain (learned_filter, then learned_prepare) is deferred:
-//          its head input goes to the warp's row slot (lane, k) in shared memory.  The other
-//          non-exact pairs run the safeguarded Newton iteration.  After the walk the warp
-//          allocates rows for its deferred pairs in the global row buffer of each head (one
-//          atomic per head and warp-block), writes their inputs there (per lane in ascending
-//          k, lanes in order) and lists the warp-block with its row bases and pair masks.
+//  rest    the walk of the universal-variable step (bia_uv_walk.cuh): short-step pairs on the spot;
+//          of the others, a pair whose fifth-order start is exact is composed, one whose start is
+//          not exact and that lies inside a head's domain (learned_filter, then learned_prepare)
+//          is deferred, the rest run the safeguarded Newton iteration.  Deferred pairs get rows in
+//          the global row buffer of each head and their warp-block a list entry: from a warp's queue, with
+//          one atomic per head for the whole queue; from a block finished on the spot
+//          (rest_block_defer), per lane in ascending k, lanes in order, with the block's pair masks.
 //  head    the rows of each head in full 256-row tiles on the tensor cores (mlp_tc.cuh), each
 //          row's guess written over its input.
 //  finish  the deferred pairs from their guesses (FP32 correction, FP64 Halley step,
@@ -107,135 +106,40 @@ constexpr size_t kListBytesPerBlock = 16 + 64 * sizeof(uint32_t) + kBatchPairs *
 // the buffer's header: the two row counts (u64) and the list length (u32), 32 bytes
 constexpr size_t kSplitHeader = 32;
 
-// Shared memory of a rest-kernel warp: its column slice (kTileSmemDoubles doubles) and 1024
-// row slots (slot lane * 32 + k: the packed head input of the lane's pair at offset k).
-constexpr size_t kRestWarpBytes = kTileSmemDoubles * sizeof(double) + 1024 * sizeof(uint32_t);
-constexpr size_t kRestSmemBytes = kTileWarps * kRestWarpBytes;
-
-// One pair of the rest kernel's walk: the universal-variable prepare and series; a non-exact
-// pair inside a head's domain is deferred (returns its head, L holds its head input), any
-// other is solved here (returns kLearnedPlain, h and its Newton iterations in it).
-__device__ __forceinline__ int rest_pair(double eps_ij, double dt, const double r[3], const double g[3],
-                                         double h[6], LearnedPair &L, int &it)
+// One pair of the rest kernel's walk that is not a short-step one: the universal-variable
+// prepare and series; a non-exact pair inside a head's domain is deferred (returns its head, x01
+// its packed head input), any other is solved here (returns kLearnedPlain, h and its Newton
+// iterations in it).  Out of line: one body for every kernel of a file, and a small walk.
+static __device__ __noinline__ int rest_pair(double eps_ij, double dt, double rx, double ry, double rz, double gx,
+                                             double gy, double gz, double *h, uint32_t *x01, int *it)
 {
-    it = 0;
+    const double r[3] = {rx, ry, rz}, g[3] = {gx, gy, gz};
+    *it = 0;
+#pragma unroll
+    for (int c = 0; c < 6; c++) h[c] = 0.0;
     const UvPair p = uv_prepare(eps_ij, r, g);
     if (dt == 0.0) return kLearnedPlain;  // h stays zero
     const UvSeries sq = uv_series(p, dt);
     if (!sq.exact && learned_filter(p, dt)) {
+        LearnedPair L;
         learned_prepare(eps_ij, dt, r, g, L);
-        if (L.kind != kLearnedPlain) return L.kind;
+        if (L.kind != kLearnedPlain) {
+            *x01 = pack_bf16(L.x0, L.x1);
+            return L.kind;
+        }
     }
     if (sq.exact) {
         uv_compose_series(p, sq, dt, r, g, h);
     } else {
         double s = uv_series_start(sq);
         double ifp = 0.0;
-        it = uv_iterate(p, dt, s, &ifp);
+        *it = uv_iterate(p, dt, s, &ifp);
         uv_compose<true>(p, s, r, g, h, ifp);
     }
     return kLearnedPlain;
 }
 
-// The non-finite pairs solved in a rest-kernel warp-block whose sums came out non-finite
-// (rare): this lane's pairs solved again, the plain ones counted one by one (the deferred
-// ones are counted where they are finished).  Out of line, so that the walk carries no copy.
-static __device__ __noinline__ int rest_block_recount(const double *si, const double *ws, bool hq, double eps_th,
-                                                      double dt, int i, int n, int bj, int lane)
-{
-    const bool diag = (i / 32 == bj);
-    const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
-    int bad = 0;
-    for (int k = k0; k <= k1; k++) {
-        const int src = (lane + k) & 31;
-        if ((!diag || k < 16 || lane < 16) && i < n && bj * 32 + src < n) {
-            const double r[3] = {si[0] - ws[0 * 32 + src], si[1] - ws[1 * 32 + src], si[2] - ws[2 * 32 + src]};
-            const double g[3] = {si[3] - ws[3 * 32 + src], si[4] - ws[4 * 32 + src], si[5] - ws[5 * 32 + src]};
-            const double eps_ij = hq ? eps_th * si[6] * ws[6 * 32 + src] : eps_th;
-            double h[6] = {0, 0, 0, 0, 0, 0};
-            LearnedPair L;
-            int it;
-            if (rest_pair(eps_ij, dt, r, g, h, L, it) == kLearnedPlain) {
-                PairCounters scratch;
-                counters_zero(scratch);
-                count_nonfinite(h, scratch);
-                bad += scratch.nonfinite;
-            }
-        }
-    }
-    return bad;
-}
-
-// The rest kernel's walk over warp-block (bi, bj) of the system x..w[0, n) (charges q,
-// coupling eps_th), with the column states and sums in the warp's slice ws and the row slots
-// wslots.  Returns the row sums racc, column sums cacc of the pairs solved here, and the
-// lane's masks of deferred pairs per head (bit k: column (lane + k) mod 32).  The pairs
-// solved here are counted as universal-variable pairs, degenerate ones included, as
-// BIA_METHOD_UNIVERSAL counts them.
-__device__ __forceinline__ void rest_block_solve(const double *x, const double *y, const double *z,
-                                                 const double *u, const double *v, const double *w,
-                                                 const double *q, int n, double eps_th, double dt, int bi, int bj,
-                                                 int lane, double *ws, uint32_t *wslots, double racc[6],
-                                                 double cacc[6], uint32_t mask[kMlpHeads], PairCounters &cnt)
-{
-    double *wacc = ws + 7 * 32;
-    const int i = bi * 32 + lane;
-    const bool diag = (bi == bj);
-    mask[kHeadEll] = mask[kHeadHyp] = 0u;
-    double si[7];
-    {
-        double sj[7];
-        load_particle(x, y, z, u, v, w, q, n, i, si);
-        load_particle(x, y, z, u, v, w, q, n, bj * 32 + lane, sj);
-#pragma unroll
-        for (int c = 0; c < 7; c++) ws[c * 32 + lane] = sj[c];
-#pragma unroll
-        for (int c = 0; c < 6; c++) wacc[c * 32 + lane] = 0.0;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int c = 0; c < 6; c++) racc[c] = 0.0;
-    counters_zero(cnt);
-    const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
-    for (int k = k0; k <= k1; k++) {
-        const int src = (lane + k) & 31;
-        const bool active = (!diag || k < 16 || lane < 16) && i < n && bj * 32 + src < n;
-        double h[6] = {0, 0, 0, 0, 0, 0};
-        if (active) {
-            const double r[3] = {si[0] - ws[0 * 32 + src], si[1] - ws[1 * 32 + src], si[2] - ws[2 * 32 + src]};
-            const double g[3] = {si[3] - ws[3 * 32 + src], si[4] - ws[4 * 32 + src], si[5] - ws[5 * 32 + src]};
-            const double eps_ij = q ? eps_th * si[6] * ws[6 * 32 + src] : eps_th;
-            LearnedPair L;
-            int it;
-            const int kind = rest_pair(eps_ij, dt, r, g, h, L, it);
-            if (kind != kLearnedPlain) {
-                mask[kind == kLearnedHyp ? kHeadHyp : kHeadEll] |= 1u << k;
-                wslots[lane * 32 + k] = pack_bf16(L.x0, L.x1);
-            } else {
-                cnt.it_uv += it;
-                if (it > kUvItMax) cnt.nonconverged++;
-                cnt.cls[kUniversal]++;
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            racc[c] += h[c];
-            wacc[c * 32 + src] += h[c];
-        }
-        __syncwarp();  // slot src is the next offset's slot of lane - 1
-    }
-#pragma unroll
-    for (int c = 0; c < 6; c++) cacc[c] = wacc[c * 32 + lane];
-    if (__any_sync(0xffffffffu, !sums_finite(racc, cacc))) {
-        double sic[7];  // a copy: passing si itself would keep it in memory for the whole walk
-#pragma unroll
-        for (int c = 0; c < 7; c++) sic[c] = si[c];
-        cnt.nonfinite += rest_block_recount(sic, ws, q != nullptr, eps_th, dt, i, n, bj, lane);
-    }
-    __syncwarp();  // the slice is reused by this warp's next block
-}
-
-// After rest_block_solve: rows for the warp-block's deferred pairs and its list entry (item:
+// Rows for a warp-block's deferred pairs (mask, the head inputs in wslots) and its list entry (item:
 // the warp-block's index for the finish kernel).  Every lane of the warp calls it.
 __device__ __forceinline__ void rest_block_defer(const LearnedRows &R, unsigned int item,
                                                  const uint32_t mask[kMlpHeads], const uint32_t *wslots, int lane)

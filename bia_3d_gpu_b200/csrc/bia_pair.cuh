@@ -1053,6 +1053,97 @@ __device__ __forceinline__ int uv_halfdisp_fast(double eps_th, double dt, const 
 }
 
 // ---------------------------------------------------------------------------
+// The short-step pair: f and g by their own power series in dt, without branches.
+//
+// With w = g dt, a = r.w/r0^2, b = |w|^2/r0^2, U = mu dt^2/r0^3 and q = b - U, the Taylor series
+// of f, g, f' and g' (from f'' = -U f/rho^3, rho^2 = |f r + g v|^2 in units of r0 and dt) are
+//   f - 1   = -(U/2) (1 + p1 + p2 + p3 + p4 + p5),      f' dt  = -U (1 + 3/2 p1 + 2 p2 + 5/2 p3 + 3 p4 + 7/2 p5),
+//   g - dt  = -(U dt/6) (1 + g1 + g2 + g3 + g4),        g' - 1 = -(U/2) (1 + 4/3 g1 + 5/3 g2 + 2 g3 + 7/3 g4),
+//   p1 = -a,  p2 = 5/4 a^2 - q/4 - U/12,  p3 = -(a/4) (7a^2 - 3q - U),
+//   p4 = a^2 (21/8 a^2 - 7/4 q - 7/12 U) + q (q/8 + U/15) + U^2/360,  p5 ~ -a p4,  and
+//   g1 = 3/2 p1,  g2 = 9/5 p2 + U/10,  g3 = 2 p3 - a U/4,  g4 ~ 15/7 p4.
+//
+// A pair is a short-step one where b + |U| <= 1.9e-7.  As a^2 <= b, the terms c_k of uv_series are
+// then inside its exactness bounds (3e-4)^k (c2 = a^2/2 - q/6, c3 = (a/2) (-9/2 c2 + a^2 + U/12),
+// c4 = a^2 (7/8 a^2 - 3/4 q - U/8) + q (3/40 q + U/120); checked on 2e7 points of the region), so
+// these pairs take no Newton iteration there either, and |a| <= 4.4e-4, p3 <= 9e-11, p4 <= 4e-14.  The
+// terms from p3 on (and the U terms of g2, which multiply a contribution of at most 2e-4 of h) are
+// formed in FP32: their rounding stays below 2e-17 of the result.  What is left out (p5 beyond -a p4,
+// g4 in g - dt, the sixth order) is below that too.  Everything from p2 down is FP64.
+//
+// It works on w (velocities times dt, so that neither dt/r0 nor its square is formed) and leaves the
+// constant factors of the half-displacement to the sums: h = 1/4 (H[0..2]) and (1/2)/dt (H[3..5]).
+// Returns false, H undefined, for any other pair: the caller takes the general solver.  Every
+// operation is written out, so that each kernel that inlines it computes the same bits; H
+// changes sign exactly with r and w.
+// ---------------------------------------------------------------------------
+struct UvFastStep {
+    double dt, dt2;
+    bool on;  // steps whose square and reciprocal are far from the limits of the type
+};
+
+__device__ __forceinline__ UvFastStep uv_fast_step(double dt)
+{
+    return {dt, dt * dt, dt > 1e-100 && dt < 1e100};
+}
+
+// 1/sqrt(x) of a normal x: the hardware approximation (relative error below 2^-19) and one step
+// of Householder's third-order iteration y (1 + e/2 + 3/8 e^2), e = 1 - x y^2.  Zero, subnormal
+// and infinite x give NaN or infinity, which uv_fast_pair's test turns away.
+__device__ __forceinline__ double rsqrt_normal(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-__dmul_rn(x, y), y, 1.0);
+    return fma(fma(e, 0.375, 0.5), __dmul_rn(y, e), y);
+}
+
+// cdt2: eps_ij dt^2
+__device__ __forceinline__ bool uv_fast_pair(double cdt2, const double r[3], const double w[3], double H[6])
+{
+    const double r2 = fma(r[2], r[2], fma(r[1], r[1], __dmul_rn(r[0], r[0])));
+    const double rw = fma(r[2], w[2], fma(r[1], w[1], __dmul_rn(r[0], w[0])));
+    const double w2 = fma(w[2], w[2], fma(w[1], w[1], __dmul_rn(w[0], w[0])));
+    const double ir = rsqrt_normal(r2);
+    const double ir2 = __dmul_rn(ir, ir);
+    const double nU = __dmul_rn(__dmul_rn(cdt2, ir), ir2);  // -U
+    const double a = __dmul_rn(rw, ir2);
+    const double q = fma(w2, ir2, nU);
+
+    // the short-step test and the terms from the third order on, in FP32
+    const float af = __double2float_rn(a), qf = __double2float_rn(q), Uf = -__double2float_rn(nU);
+    const bool ok = __fadd_rn(__fadd_rn(qf, Uf), fabsf(Uf)) <= 1.9e-7f;
+    const float A = __fmul_rn(af, af);
+    const float p3 = __fmul_rn(__fmul_rn(-0.25f, af), __fmaf_rn(7.0f, A, __fmaf_rn(-3.0f, qf, -Uf)));
+    const float p4 = __fmaf_rn(A, __fmaf_rn(2.625f, A, __fmaf_rn(-1.75f, qf, __fmul_rn(-7.0f / 12.0f, Uf))),
+                               __fmaf_rn(qf, __fmaf_rn(0.125f, qf, __fmul_rn(1.0f / 15.0f, Uf)),
+                                         __fmul_rn(Uf, __fmul_rn(1.0f / 360.0f, Uf))));
+    const float p45 = __fmaf_rn(-af, p4, p4);
+    const float cf = __fadd_rn(p3, p45);
+    const float cfd = __fmaf_rn(2.5f, p3, __fmul_rn(3.0f, p45));
+    const float aU = __fmul_rn(af, Uf);
+    const float cg = __fmaf_rn(2.0f / 3.0f, p3, __fmaf_rn(-0.25f / 3.0f, aU, __fmul_rn(0.1f / 3.0f, Uf)));
+    const float cgd = __fmaf_rn(2.0f, p3, __fmaf_rn(2.5f, p4, __fmaf_rn(-0.25f, aU, __fmul_rn(1.0f / 12.0f, Uf))));
+
+    // the leading terms in FP64, the small ones first (a multiply-add with one constant operand each, so
+    // that no constant waits in a register): the four series, that of g - dt over 3, of g' - 1 over 2
+    const double p2 = fma(1.25, __dmul_rn(a, a), fma(-0.25, q, __dmul_rn(1.0 / 12.0, nU)));
+    const double sf = __dadd_rn(__dsub_rn(__dadd_rn(p2, (double)cf), a), 1.0);
+    const double sfd = __dadd_rn(fma(2.0, fma(-0.75, a, p2), (double)cfd), 1.0);
+    const double sg = __dadd_rn(fma(0.6, p2, fma(-0.5, a, (double)cg)), 1.0 / 3.0);
+    const double sgd = __dadd_rn(__dsub_rn(fma(1.5, p2, (double)cgd), a), 0.5);
+    const double F = __dmul_rn(nU, sf), G = __dmul_rn(nU, sg);
+    const double Fd = __dmul_rn(nU, sfd), Gd = __dmul_rn(nU, sgd);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        H[k] = fma(F, r[k], __dmul_rn(G, w[k]));
+        H[3 + k] = fma(Fd, r[k], __dmul_rn(Gd, w[k]));
+    }
+    return ok;
+}
+
+
+// ---------------------------------------------------------------------------
 // One pair: frame, classification, solve, half-displacement (bia/bia.f90:141-191).
 // Returns the half-displacement in h[6] = (dX, dY, dZ, dU, dV, dW)/2 terms.
 // ---------------------------------------------------------------------------
@@ -1097,7 +1188,7 @@ __device__ __forceinline__ bool pair_degenerate(const double r[3], const double 
     return gsq == 0.0 || (L0 * L0 + L1 * L1 + L2 * L2) == 0.0;
 }
 
-// M: the compiled method (kMethodRkf, kMethodAlg, kMethodUniversal); each kernel is
+// M: the compiled method (kMethodRkf or kMethodAlg); each kernel is
 // instantiated per method so it carries only that method's code and registers.
 constexpr int kMethodRkf = 0, kMethodAlg = 1, kMethodUniversal = 2, kMethodLearned = 3;
 
@@ -1169,20 +1260,11 @@ __device__ __forceinline__ void alg_rare_pair(const PairParams &P, double eps_ij
     }
 }
 
-// kCountNonfinite false (universal variables and RKF45 only): the caller counts the
-// non-finite half-displacements itself (once per warp-block from its sums, see
-// warp_block_solve_uv).
-template <int M, bool kCountNonfinite = true>
+template <int M>
 __device__ __forceinline__ void pair_halfdisp(const PairParams &P, double eps_ij, const double r[3],
                                               const double g[3], double h[6], PairCounters &cnt)
 {
-    if (M == kMethodUniversal) {
-        const int it = uv_halfdisp_fast(eps_ij, P.dt, r, g, h);
-        cnt.it_uv += it;
-        if (it > kUvItMax) cnt.nonconverged++;
-        cnt.cls[kUniversal]++;
-        if (kCountNonfinite) count_nonfinite(h, cnt);
-    } else if (M == kMethodAlg) {
+    if (M == kMethodAlg) {
         const int c = alg_classify(eps_ij, r, g);
         if (c == kClsUv || c == kClsDeg) {
             alg_rare_pair(P, eps_ij, r, g, h, cnt, c);
@@ -1220,19 +1302,8 @@ __device__ __forceinline__ void pair_halfdisp(const PairParams &P, double eps_ij
         cnt.rkf_steps += nacc;
         if (fabs(error) > P.err) cnt.nonconverged++;
         compose_halfdisp(P, g, e_xi, e_eta, YZ, YN, h);
-        if (kCountNonfinite) count_nonfinite(h, cnt);
+        count_nonfinite(h, cnt);
     }
-}
-
-// A warp-block's sums are finite exactly when every half-displacement added into them is (a
-// NaN stays NaN and an infinity stays infinite or turns NaN), so the walks test the lane's
-// row and column sums once per block instead of each pair.
-__device__ __forceinline__ bool sums_finite(const double racc[6], const double cacc[6])
-{
-    bool ok = true;
-#pragma unroll
-    for (int c = 0; c < 6; c++) ok = ok && isfinite(racc[c]) && isfinite(cacc[c]);
-    return ok;
 }
 
 }  // namespace bia

@@ -34,6 +34,7 @@
 #include "bia_learned_block.cuh"
 #include "bia_pair.cuh"
 #include "bia_tiles.cuh"
+#include "bia_uv_walk.cuh"
 #include "mlp_tc.cuh"
 
 namespace bia {
@@ -57,11 +58,10 @@ struct StepArgs {
     LearnedRows R;
 };
 
-// Each warp solves warp-blocks t = (its global warp index) + k * (warps in the grid): one
-// block per warp when the grid covers every block, several in a persistent grid (the
-// universal-variable and split-step rest kernels launch one resident grid, kPersistentCtas
-// CTAs per SM).  The counters are summed per warp in registers and flushed every
-// kFlushBlocks blocks: one set of atomics per warp instead of one per block.
+// ALG and RKF45: each warp solves warp-blocks t = (its global warp index) + k * (warps in the grid), one
+// block per warp when the grid covers every block.  The counters are summed per warp in
+// registers and flushed every kFlushBlocks blocks: one set of atomics per warp instead of one
+// per block.
 template <bool kDeterministic, int M>
 __global__ void __launch_bounds__(kThreads, TileOccupancy<M>::kMinBlocks) bia_pair_tiles_kernel(const StepArgs A)
 {
@@ -249,6 +249,41 @@ static int ilog2_bucket(int n)
     return b;
 }
 
+// The warp-blocks of a single system for uv_walk_blocks.
+struct StepItems {
+    const StepArgs &A;
+    __device__ __forceinline__ WalkBlock block(long long tl) const
+    {
+        WalkBlock B;
+        const long long t = A.t0 + tl;
+        warp_block_coords(t, B.bi, B.bj);
+        B.sys = 0;
+        B.item = (unsigned int)t;
+        return B;
+    }
+    __device__ __forceinline__ WalkSystem system(int) const
+    {
+        return {A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, A.eps_th, A.part, (size_t)A.npad};
+    }
+};
+
+// The universal-variable step (kRest false) and the split learned step's first kernel, the rest pass
+// (kRest true: a pair that is not exact by series and inside a head's domain is deferred, its head
+// input to the rows, its block to the list): a persistent grid of kPersistentCtas CTAs per SM
+// (128 registers a thread; three or four CTAs with the registers that leaves are slower, 4.36 to 4.62
+// against 4.10 ms a step on plummer_32768), the counters flushed once per warp.  Deterministic
+// mode writes every partial slot here.
+template <bool kDeterministic, bool kRest>
+__global__ void __launch_bounds__(kThreads, kPersistentCtas) bia_pair_walk_kernel(const StepArgs A)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    WalkCounts c = {0, 0, 0, 0};
+    uv_walk_blocks<kDeterministic, kRest>(StepItems{A}, (long long)blockIdx.x * kWarpsPerBlock + warp,
+                                          (long long)gridDim.x * kWarpsPerBlock, A.nwb, A.P.dt,
+                                          warp * walk_warp_doubles<kRest>(), A.R, c);
+    walk_flush_counts(c, A.stats, lane);
+}
+
 template <bool kDeterministic>
 static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st, int tuned = -1)
 {
@@ -267,11 +302,11 @@ static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st
     }
     switch (A.P.method) {
     case kMethodRkf:
-        bia_pair_tiles_kernel<kDeterministic, kMethodRkf><<<(unsigned)grid, kThreads, 0, st>>>(A);
+        bia_pair_tiles_kernel<kDeterministic, kMethodRkf><<<(unsigned)grid, kThreads, kSliceBytes, st>>>(A);
         break;
     case kMethodUniversal:
-        bia_pair_tiles_kernel<kDeterministic, kMethodUniversal>
-            <<<(unsigned)persistent_grid(grid), kThreads, 0, st>>>(A);
+        bia_pair_walk_kernel<kDeterministic, false>
+            <<<(unsigned)persistent_grid(grid), kThreads, walk_smem_bytes<false>(kWarpsPerBlock), st>>>(A);
         break;
     default:
         bia_pair_tiles_kernel<kDeterministic, kMethodAlg><<<(unsigned)grid, kThreads, 0, st>>>(A);
@@ -334,55 +369,6 @@ __global__ void __launch_bounds__(kMlpThreads, 2) bia_pair_learned_kernel(const 
     if (!live) return;  // warp-uniform; no barrier follows
     flush_counters(cnt, A.stats, lane);
     add_learned_sums<kDeterministic>(A, bi, bj, lane, racc, cacc, true);
-}
-
-// Split learned step, first kernel (rest_block_solve, rest_block_defer): every warp-block's
-// pairs except the deferred ones, whose head inputs go to the rows and whose warp-blocks are
-// listed.  Deterministic mode writes every partial slot here; the finish kernel adds onto
-// them.  Two CTAs per SM (kPersistentCtas): at three the filter spills registers inside the
-// rotation loop.  A persistent grid with the counters flushed per warp, as
-// bia_pair_tiles_kernel; dynamic shared memory: each warp's column slice and row slots.
-// Warps per CTA of the rest kernel.  At 112 registers the register file would hold 18 warps
-// per SM, but CTAs of 9 (96 registers, small spills) or 10 warps (92 registers) are slower:
-// 6.45 and 6.50 against 5.61 ms for the learned pair kernels on plummer_32768.
-#ifndef BIA_REST_WARPS
-#define BIA_REST_WARPS 8
-#endif
-constexpr int kRestWarps = BIA_REST_WARPS;
-constexpr size_t kRestKernelSmemBytes = kRestWarps * kRestWarpBytes;
-
-template <bool kDeterministic>
-__global__ void __launch_bounds__(kRestWarps * 32, kPersistentCtas) bia_pair_rest_kernel(const StepArgs A)
-{
-    extern __shared__ __align__(16) uint8_t rest_smem[];
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    double *ws = reinterpret_cast<double *>(rest_smem + warp * kRestWarpBytes);
-    uint32_t *wslots = reinterpret_cast<uint32_t *>(rest_smem + warp * kRestWarpBytes +
-                                                    kTileSmemDoubles * sizeof(double));
-    PairCounters tot;
-    counters_zero(tot);
-    int nblk = 0;
-    for (long long tl = (long long)blockIdx.x * kRestWarps + warp; tl < A.nwb;
-         tl += (long long)gridDim.x * kRestWarps) {  // warp-uniform
-        const long long t = A.t0 + tl;
-        int bi, bj;
-        warp_block_coords(t, bi, bj);
-        double racc[6], cacc[6];
-        uint32_t mask[kMlpHeads];
-        PairCounters cnt;
-        rest_block_solve(A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, A.eps_th, A.P.dt, bi, bj, lane, ws, wslots, racc,
-                         cacc, mask, cnt);
-        counters_add(tot, cnt);
-        if (++nblk == kFlushBlocks) {
-            flush_counters(tot, A.stats, lane);
-            counters_zero(tot);
-            nblk = 0;
-        }
-        add_learned_sums<kDeterministic>(A, bi, bj, lane, racc, cacc, true);
-        rest_block_defer(A.R, (unsigned int)t, mask, wslots, lane);
-    }
-    if (nblk > 0) flush_counters(tot, A.stats, lane);
 }
 
 // Split learned step, second kernel: the rows of both heads on the tensor cores (persistent
@@ -510,10 +496,10 @@ static int learned_kernel_setup()
                                         bytes) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(bia_pair_learned_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         bytes) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_rest_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kRestKernelSmemBytes) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_rest_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kRestKernelSmemBytes) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_walk_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)walk_smem_bytes<true>(kWarpsPerBlock)) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_walk_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)walk_smem_bytes<true>(kWarpsPerBlock)) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(bia_pair_learned_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         hbytes) == cudaSuccess;
         // the largest shared-memory carveout, so that the occupancy query sees what the
@@ -554,8 +540,9 @@ static int launch_pair_learned(const StepArgs &A, cudaStream_t st)
     }
     // the row counts of both heads and the list length start at zero
     if (cudaMemsetAsync(A.R.counts, 0, kSplitHeader, st) != cudaSuccess) return BIA_ERR_CUDA;
-    const long long rgrid = persistent_grid((A.nwb + kRestWarps - 1) / kRestWarps);
-    bia_pair_rest_kernel<kDeterministic><<<(unsigned)rgrid, kRestWarps * 32, kRestKernelSmemBytes, st>>>(A);
+    const long long rgrid = persistent_grid((A.nwb + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    bia_pair_walk_kernel<kDeterministic, true>
+        <<<(unsigned)rgrid, kThreads, walk_smem_bytes<true>(kWarpsPerBlock), st>>>(A);
     launch_learned_head(A.R, A.heads, A.stats, lgrid, st);
     const long long fgrid = persistent_grid((A.nwb + kWarpsPerBlock - 1) / kWarpsPerBlock);
     bia_pair_learned_finish_kernel<kDeterministic><<<(unsigned)fgrid, kThreads, 0, st>>>(A);

@@ -18,12 +18,9 @@ namespace bia {
 
 // Resident CTAs per SM each method's 8-warp kernel is compiled for (register budget
 // 65536 / (256 threads * blocks)): ALG 3 (<= 85 registers, measured fastest on the
-// mixed-class Coulomb workload), universal variables 2 and RKF45 2 (<= 128).
+// mixed-class Coulomb workload) and RKF45 2 (<= 128).
 #ifndef BIA_ALG_MIN_BLOCKS
 #define BIA_ALG_MIN_BLOCKS 3
-#endif
-#ifndef BIA_UV_MIN_BLOCKS
-#define BIA_UV_MIN_BLOCKS 2  // 3 spills in the rotation loop: 9.4 ms vs 8.6 ms at n = 32768
 #endif
 // RKF45: the shared-memory column walk at two CTAs per SM (128 registers; 600 B of spills
 // around the out-of-line pair integrator) measured 184 ms per Coulomb step at n = 32768
@@ -38,7 +35,6 @@ namespace bia {
 template <int M> struct TileOccupancy { static constexpr int kMinBlocks = 1; };
 template <> struct TileOccupancy<kMethodRkf> { static constexpr int kMinBlocks = BIA_RKF_MIN_BLOCKS; };
 template <> struct TileOccupancy<kMethodAlg> { static constexpr int kMinBlocks = BIA_ALG_MIN_BLOCKS; };
-template <> struct TileOccupancy<kMethodUniversal> { static constexpr int kMinBlocks = BIA_UV_MIN_BLOCKS; };
 
 __device__ __forceinline__ void warp_block_coords(long long t, int &bi, int &bj)
 {
@@ -382,61 +378,98 @@ __device__ __forceinline__ void phase_block_solve(const double *x, const double 
     }
 }
 
-// Universal-variable warp-block: lanes walk the rotation offsets as in warp_block_solve,
-// with the column states and the column sums in the warp's shared slice instead of
-// registers and shuffles.  Lane l adds its pair at offset k into column slot (l + k) mod 32,
-// a different slot on every lane, so the slots take their pairs in ascending k, the order
-// of the shuffle walk: the sums are bitwise the same.  Measured at n = 32768: 6.48 ms
-// against 6.79 ms for the shuffle walk (100 instead of 118 registers, no shuffles).
-// The non-finite pairs of a warp-block whose sums came out non-finite (rare): this lane's
-// pairs solved again, counted one by one.  Out of line, so that the walk carries no copy.
-template <int M>
-static __device__ __noinline__ int uv_block_recount(const PairParams &P, const double *si, const double *ws,
-                                                    bool hq, double eps_th, int i, int n, int bj, int lane)
+constexpr size_t kSliceBytes = kTileWarps * kTileSmemDoubles * sizeof(double);
+
+// The column slice of the universal-variable, rest and RKF45 walks: the column states as three
+// double2 rows (x, y), (z, u), (v, w) of 32 slots and the charges, then the column sums as three
+// double2 rows.  A pair reads its column and adds its sums with three 16-byte accesses each,
+// half the shared-memory instructions of one row per component (lane l at slot (l + k) mod 32: no
+// bank conflicts either way).
+__device__ __forceinline__ double2 *slice_cols(double *ws) { return reinterpret_cast<double2 *>(ws); }
+__device__ __forceinline__ const double2 *slice_cols(const double *ws) { return reinterpret_cast<const double2 *>(ws); }
+__device__ __forceinline__ double2 *slice_sums(double *ws) { return reinterpret_cast<double2 *>(ws + 7 * 32); }
+
+__device__ __forceinline__ void slice_states(double *ws, int lane, const double sj[7])
 {
-    const bool diag = (i / 32 == bj);
-    const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
-    int bad = 0;
-    for (int k = k0; k <= k1; k++) {
-        const int src = (lane + k) & 31;
-        if ((!diag || k < 16 || lane < 16) && i < n && bj * 32 + src < n) {
-            const double r[3] = {si[0] - ws[0 * 32 + src], si[1] - ws[1 * 32 + src], si[2] - ws[2 * 32 + src]};
-            const double g[3] = {si[3] - ws[3 * 32 + src], si[4] - ws[4 * 32 + src], si[5] - ws[5 * 32 + src]};
-            const double eps_ij = hq ? eps_th * si[6] * ws[6 * 32 + src] : eps_th;
-            double h[6];
-            PairCounters scratch;
-            counters_zero(scratch);
-            pair_halfdisp<M, true>(P, eps_ij, r, g, h, scratch);
-            bad += scratch.nonfinite;
-        }
-    }
-    return bad;
+    double2 *col = slice_cols(ws);
+#pragma unroll
+    for (int c = 0; c < 3; c++) col[c * 32 + lane] = make_double2(sj[2 * c], sj[2 * c + 1]);
+    ws[6 * 32 + lane] = sj[6];
 }
 
-template <int M = kMethodUniversal>
-__device__ __forceinline__ void warp_block_solve_uv(const double *x, const double *y, const double *z,
-                                                    const double *u, const double *v, const double *w,
-                                                    const double *q, int n, double eps_th, const PairParams &P,
-                                                    int bi, int bj, int lane, double racc[6], double cacc[6],
-                                                    PairCounters &cnt)
+// the states, and the sums from zero
+__device__ __forceinline__ void slice_fill(double *ws, int lane, const double sj[7])
 {
-    // universal variables: the non-finite pairs counted from the block's sums (one test per
-    // block instead of six per pair); RKF45 pairs are costly enough to keep the per-pair count
-    constexpr bool kBlockCheck = (M == kMethodUniversal);
-    __shared__ double s_uv[kTileWarps][kTileSmemDoubles];
-    double *ws = s_uv[(threadIdx.x >> 5) % kTileWarps];
-    double *wacc = ws + 7 * 32;
-    const int i = bi * 32 + lane;
-    double si[7];
-    {
-        double sj[7];
-        load_particle(x, y, z, u, v, w, q, n, i, si);
-        load_particle(x, y, z, u, v, w, q, n, bj * 32 + lane, sj);
+    slice_states(ws, lane, sj);
+    double2 *acc = slice_sums(ws);
 #pragma unroll
-        for (int c = 0; c < 7; c++) ws[c * 32 + lane] = sj[c];
+    for (int c = 0; c < 3; c++) acc[c * 32 + lane] = make_double2(0.0, 0.0);
+}
+
+// relative state of row si against column slot src
+__device__ __forceinline__ void slice_diff(const double *ws, int src, const double *si, double r[3], double g[3])
+{
+    const double2 *col = slice_cols(ws);
+    const double2 xy = col[src], zu = col[32 + src], vw = col[64 + src];
+    r[0] = si[0] - xy.x;
+    r[1] = si[1] - xy.y;
+    r[2] = si[2] - zu.x;
+    g[0] = si[3] - zu.y;
+    g[1] = si[4] - vw.x;
+    g[2] = si[5] - vw.y;
+}
+
+// the same and the pair's coupling
+__device__ __forceinline__ double slice_pair(const double *ws, int src, const double *si, bool hq, double eps_th,
+                                             double r[3], double g[3])
+{
+    slice_diff(ws, src, si, r, g);
+    return hq ? eps_th * si[6] * ws[6 * 32 + src] : eps_th;
+}
+
+__device__ __forceinline__ void slice_add(double *ws, int src, const double h[6], double racc[6])
+{
+    double2 *acc = slice_sums(ws);
 #pragma unroll
-        for (int c = 0; c < 6; c++) wacc[c * 32 + lane] = 0.0;
+    for (int c = 0; c < 3; c++) {
+        racc[2 * c] += h[2 * c];
+        racc[2 * c + 1] += h[2 * c + 1];
+        double2 t = acc[c * 32 + src];
+        t.x += h[2 * c];
+        t.y += h[2 * c + 1];
+        acc[c * 32 + src] = t;
     }
+}
+
+// the lane's own column sums
+__device__ __forceinline__ void slice_sums_of(double *ws, int lane, double cacc[6])
+{
+    const double2 *acc = slice_sums(ws);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        cacc[2 * c] = acc[c * 32 + lane].x;
+        cacc[2 * c + 1] = acc[c * 32 + lane].y;
+    }
+}
+
+// RKF45 warp-block: lanes walk the rotation offsets with the column states and the column sums in the
+// warp's slice of the dynamic shared memory (kSliceBytes per CTA).  Lane l adds its pair at offset k
+// into column slot (l + k) mod 32, a different slot on every lane.
+extern __shared__ __align__(16) double warp_slices[];
+
+__device__ __forceinline__ void warp_block_solve_rkf(const double *x, const double *y, const double *z,
+                                                     const double *u, const double *v, const double *w,
+                                                     const double *q, int n, double eps_th, const PairParams &P,
+                                                     int bi, int bj, int lane, double racc[6], double cacc[6],
+                                                     PairCounters &cnt)
+{
+    double *ws = warp_slices + (int)(threadIdx.x >> 5) * kTileSmemDoubles;
+    const int i = bi * 32 + lane;
+    const bool hq = q != nullptr;
+    double si[7], sj[7];
+    load_particle(x, y, z, u, v, w, q, n, i, si);
+    load_particle(x, y, z, u, v, w, q, n, bj * 32 + lane, sj);
+    slice_fill(ws, lane, sj);
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < 6; c++) racc[c] = 0.0;
@@ -449,26 +482,14 @@ __device__ __forceinline__ void warp_block_solve_uv(const double *x, const doubl
         const bool active = (!diag || k < 16 || lane < 16) && i < n && bj * 32 + src < n;
         double h[6] = {0, 0, 0, 0, 0, 0};
         if (active) {
-            const double r[3] = {si[0] - ws[0 * 32 + src], si[1] - ws[1 * 32 + src], si[2] - ws[2 * 32 + src]};
-            const double g[3] = {si[3] - ws[3 * 32 + src], si[4] - ws[4 * 32 + src], si[5] - ws[5 * 32 + src]};
-            const double eps_ij = q ? eps_th * si[6] * ws[6 * 32 + src] : eps_th;
-            pair_halfdisp<M, !kBlockCheck>(P, eps_ij, r, g, h, cnt);
+            double r[3], g[3];
+            const double eps_ij = slice_pair(ws, src, si, hq, eps_th, r, g);
+            pair_halfdisp<kMethodRkf>(P, eps_ij, r, g, h, cnt);
         }
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            racc[c] += h[c];
-            wacc[c * 32 + src] += h[c];
-        }
+        slice_add(ws, src, h, racc);
         __syncwarp();  // slot src is the next offset's slot of lane - 1
     }
-#pragma unroll
-    for (int c = 0; c < 6; c++) cacc[c] = wacc[c * 32 + lane];
-    if (kBlockCheck && __any_sync(0xffffffffu, !sums_finite(racc, cacc))) {
-        double sic[7];  // a copy: passing si itself would keep it in memory for the whole walk
-#pragma unroll
-        for (int c = 0; c < 7; c++) sic[c] = si[c];
-        cnt.nonfinite += uv_block_recount<M>(P, sic, ws, q != nullptr, eps_th, i, n, bj, lane);
-    }
+    slice_sums_of(ws, lane, cacc);
     __syncwarp();  // the slice is reused by this warp's next block
 }
 
@@ -525,8 +546,8 @@ __device__ __forceinline__ void warp_block_solve(const double *x, const double *
         warp_block_solve_compact(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
         return;
     }
-    if (M == kMethodUniversal || (M == kMethodRkf && BIA_RKF_SMEM)) {
-        warp_block_solve_uv<M>(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
+    if (M == kMethodRkf && BIA_RKF_SMEM) {
+        warp_block_solve_rkf(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
         return;
     }
     const unsigned full = 0xffffffffu;
