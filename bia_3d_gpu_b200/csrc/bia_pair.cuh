@@ -617,63 +617,148 @@ struct Fehlberg {
                             DA5 = 1.0 / 50, DA6 = 2.0 / 55;
 };
 
-__device__ __forceinline__ void moon2d(double eps_th, const double Y[4], double F[4])
+// 1/sqrt(x) of a normal x: the hardware approximation and one step
+// of Householder's third-order iteration y (1 + e/2 + 3/8 e^2), e = 1 - x y^2 (measured
+// at most 2^-19.04 over 1e9 values; the next term, 5/16 e^3, is below 3e-18).  Zero, subnormal
+// and infinite x give NaN or infinity: its callers test for them.
+__device__ __forceinline__ double rsqrt_normal(double x)
 {
-    const double rsq = Y[0] * Y[0] + Y[1] * Y[1];
-    const double aaa = eps_th / (rsq * sqrt(rsq));
-    F[0] = Y[2];
-    F[1] = Y[3];
-    F[2] = Y[0] * aaa;
-    F[3] = Y[1] * aaa;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-__dmul_rn(x, y), y, 1.0);
+    return fma(fma(e, 0.375, 0.5), __dmul_rn(y, e), y);
 }
 
-// bia/find_dXYUV_RKF.f90:150-157 fehl on 4 equations; er written when want_er.
-__device__ __forceinline__ void fehl4(double eps_th, double h, const double y0[4], double yn[4],
-                                      double er[4], bool want_er)
+// c x^(-3/2) of a normal x from the same approximation y, whose square is exact (its low half is zero):
+// c y^3 (1 + 3/2 e + 15/8 e^2), e = 1 - x y^2; the next term, 35/16 e^3, is below 3e-17.
+__device__ __forceinline__ double scaled_rsqrt3_normal(double c, double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double y2 = y * y;
+    const double e = fma(-x, y2, 1.0);
+    const double c3 = (c * y) * y2;
+    return fma(c3 * e, fma(e, 1.875, 1.5), c3);
+}
+
+// Acceleration (ax, ay) = eps (x, y) / r^3 of moon_2D.  kNormal: eps r^-3 from one reciprocal square
+// root (x^2 + y^2 a normal number), at about half the FP64 instructions of the reference's
+// eps / (rsq sqrt(rsq)) (bia/find_dXYUV_RKF.f90:15-23), which the other form keeps.
+template <bool kNormal>
+__device__ __forceinline__ void moon_acc(double eps_th, double x, double y, double &ax, double &ay)
+{
+    const double rsq = x * x + y * y;
+    double aaa;
+    if (kNormal) {
+        aaa = scaled_rsqrt3_normal(eps_th, rsq);
+    } else {
+        aaa = eps_th / (rsq * sqrt(rsq));
+    }
+    ax = x * aaa;
+    ay = y * aaa;
+}
+
+// bia/find_dXYUV_RKF.f90:150-157 fehl on the planar state (x, y, u, v) from y0 with its acceleration
+// a1 = (ax, ay); er written when kWantEr.  A position's derivative is the stage's velocity
+// u0 + h sum_m B_sm a_m, so the position of stage s is x0 + c_s h u0 + h^2 sum_m N_sm a_m with
+// N = B B (and GA B, DA B for the new position and its error): the accelerations are all that is
+// kept, no stage velocity is formed, and a step takes 62 operations for its sums instead of 100.
+struct FehlbergNested {
+    using F = Fehlberg;
+    static constexpr double N31 = F::B32 * F::B21;
+    static constexpr double N41 = F::B42 * F::B21 + F::B43 * F::B31, N42 = F::B43 * F::B32;
+    static constexpr double N51 = F::B52 * F::B21 + F::B53 * F::B31 + F::B54 * F::B41,
+                            N52 = F::B53 * F::B32 + F::B54 * F::B42, N53 = F::B54 * F::B43;
+    static constexpr double N61 = F::B62 * F::B21 + F::B63 * F::B31 + F::B64 * F::B41 + F::B65 * F::B51,
+                            N62 = F::B63 * F::B32 + F::B64 * F::B42 + F::B65 * F::B52,
+                            N63 = F::B64 * F::B43 + F::B65 * F::B53, N64 = F::B65 * F::B54;
+    static constexpr double G1 = F::GA3 * F::B31 + F::GA4 * F::B41 + F::GA5 * F::B51 + F::GA6 * F::B61,
+                            G2 = F::GA3 * F::B32 + F::GA4 * F::B42 + F::GA5 * F::B52 + F::GA6 * F::B62,
+                            G3 = F::GA4 * F::B43 + F::GA5 * F::B53 + F::GA6 * F::B63,
+                            G4 = F::GA5 * F::B54 + F::GA6 * F::B64, G5 = F::GA6 * F::B65;
+    static constexpr double D1 = F::DA3 * F::B31 + F::DA4 * F::B41 + F::DA5 * F::B51 + F::DA6 * F::B61,
+                            D2 = F::DA3 * F::B32 + F::DA4 * F::B42 + F::DA5 * F::B52 + F::DA6 * F::B62,
+                            D3 = F::DA4 * F::B43 + F::DA5 * F::B53 + F::DA6 * F::B63,
+                            D4 = F::DA5 * F::B54 + F::DA6 * F::B64, D5 = F::DA6 * F::B65;
+};
+
+template <bool kNormal, bool kWantEr>
+__device__ __forceinline__ void fehl4(double eps_th, double h, const double y0[4], const double a1[2], double yn[4],
+                                      double er[4])
 {
     using F = Fehlberg;
-    double k1[4], k2[4], k3[4], k4[4], k5[4], k6[4], w[4];
-    moon2d(eps_th, y0, k1);
+    using N = FehlbergNested;
+    const double h2 = h * h;
+    const double hu[2] = {h * y0[2], h * y0[3]};
+    double a2[2], a3[2], a4[2], a5[2], a6[2], p[2];
 #pragma unroll
-    for (int i = 0; i < 4; i++) w[i] = y0[i] + h * F::B21 * k1[i];
-    moon2d(eps_th, w, k2);
+    for (int i = 0; i < 2; i++) p[i] = fma(F::AL2, hu[i], y0[i]);
+    moon_acc<kNormal>(eps_th, p[0], p[1], a2[0], a2[1]);
 #pragma unroll
-    for (int i = 0; i < 4; i++) w[i] = y0[i] + h * (F::B31 * k1[i] + F::B32 * k2[i]);
-    moon2d(eps_th, w, k3);
+    for (int i = 0; i < 2; i++) p[i] = fma(h2, N::N31 * a1[i], fma(F::AL3, hu[i], y0[i]));
+    moon_acc<kNormal>(eps_th, p[0], p[1], a3[0], a3[1]);
 #pragma unroll
-    for (int i = 0; i < 4; i++) w[i] = y0[i] + h * (F::B41 * k1[i] + F::B42 * k2[i] + F::B43 * k3[i]);
-    moon2d(eps_th, w, k4);
+    for (int i = 0; i < 2; i++) p[i] = fma(h2, N::N41 * a1[i] + N::N42 * a2[i], fma(F::AL4, hu[i], y0[i]));
+    moon_acc<kNormal>(eps_th, p[0], p[1], a4[0], a4[1]);
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        w[i] = y0[i] + h * (F::B51 * k1[i] + F::B52 * k2[i] + F::B53 * k3[i] + F::B54 * k4[i]);
-    moon2d(eps_th, w, k5);
+    for (int i = 0; i < 2; i++)
+        p[i] = fma(h2, N::N51 * a1[i] + N::N52 * a2[i] + N::N53 * a3[i], y0[i] + hu[i]);
+    moon_acc<kNormal>(eps_th, p[0], p[1], a5[0], a5[1]);
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        w[i] = y0[i] + h * (F::B61 * k1[i] + F::B62 * k2[i] + F::B63 * k3[i] + F::B64 * k4[i] +
-                            F::B65 * k5[i]);
-    moon2d(eps_th, w, k6);
+    for (int i = 0; i < 2; i++)
+        p[i] = fma(h2, N::N61 * a1[i] + N::N62 * a2[i] + N::N63 * a3[i] + N::N64 * a4[i],
+                   fma(F::AL6, hu[i], y0[i]));
+    moon_acc<kNormal>(eps_th, p[0], p[1], a6[0], a6[1]);
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        yn[i] = y0[i] + h * (F::GA1 * k1[i] + F::GA3 * k3[i] + F::GA4 * k4[i] + F::GA5 * k5[i] +
-                             F::GA6 * k6[i]);
-    if (want_er) {
+    for (int i = 0; i < 2; i++) {
+        yn[i] = y0[i] + fma(h2, N::G1 * a1[i] + N::G2 * a2[i] + N::G3 * a3[i] + N::G4 * a4[i] + N::G5 * a5[i], hu[i]);
+        yn[2 + i] = fma(h, F::GA1 * a1[i] + F::GA3 * a3[i] + F::GA4 * a4[i] + F::GA5 * a5[i] + F::GA6 * a6[i],
+                        y0[2 + i]);
+    }
+    if (kWantEr) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            er[i] = h * (F::DA1 * k1[i] + F::DA3 * k3[i] + F::DA4 * k4[i] + F::DA5 * k5[i] +
-                         F::DA6 * k6[i]);
+        for (int i = 0; i < 2; i++) {
+            er[i] = h2 * (N::D1 * a1[i] + N::D2 * a2[i] + N::D3 * a3[i] + N::D4 * a4[i] + N::D5 * a5[i]);
+            er[2 + i] = h * (F::DA1 * a1[i] + F::DA3 * a3[i] + F::DA4 * a4[i] + F::DA5 * a5[i] + F::DA6 * a6[i]);
+        }
     }
 }
 
-static __device__ __noinline__ int rkf_pair(double eps_th, double xe, double relerr, double abserr,
-                                     const double YZ[4], double YN[4], double *error, int *nacc)
+// x^(1/5) of the step control: an FP32 power and two Newton steps on y^-5 = 1/x in FP64 (quadratic: 1e-6,
+// 3e-12, 3e-23 before rounding), where x is well inside FP32's range; else pow.
+__device__ __forceinline__ double fifth_root(double x)
+{
+    if (!(x > 1e-30 && x < 1e30)) return pow(x, 0.2);
+    double y = (double)powf((float)x, -0.2f);  // x^(-1/5): y (6 - x y^5) / 5
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double y2 = y * y;
+        y = y * fma(-0.2 * x, y2 * y2 * y, 1.2);
+    }
+    const double y2 = y * y;
+    return x * (y2 * y2);  // x x^(-4/5)
+}
+
+// The step with its control, two copies of the Fehlberg step in all (the low step, tried and, to the
+// end, repeated; the half step): four inlined copies fetched more instructions than the SM's caches
+// hold.  What bounds it: the FP64 pipe (67 % busy, 2225 instructions a pair of four steps) and the
+// latency of a stage's dependent chain at 16 warps per SM; 24 warps spill and are no faster (5.98 against 5.79
+// ms).  Coulomb step at n = 8191: 12.8 ms with divisions and roots, 6.9 with reciprocal square
+// roots, fifth roots and one division for the error norm, 6.0 without stage velocities, 5.8 with
+// two copies.  kNormal: r^2 stays a normal number over the step (rkf_pair decides by the pair's
+// initial state).
+template <bool kNormal>
+static __device__ __noinline__ int rkf_pair_form(double eps_th, double xe, double relerr, double abserr,
+                                                 const double YZ[4], double YN[4], double *error, int *nacc)
 {
     const int itemax = 100000;
     const double epsmin = 1e-15;
-    double yh0[4], yl0[4], yln[4], yhn[4], er[4], ymid[4];
+    double yh0[4], yl0[4], yln[4], yhn[4], er[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) { yh0[i] = YZ[i]; yl0[i] = YZ[i]; yhn[i] = YZ[i]; }
-    double f0[4];
-    moon2d(eps_th, yl0, f0);
+    double al[2];  // the acceleration of yl0
+    moon_acc<kNormal>(eps_th, yl0[0], yl0[1], al[0], al[1]);
+    const double f0[4] = {yl0[2], yl0[3], al[0], al[1]};
     double toldy = 1.7976931348623157e308;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -682,50 +767,83 @@ static __device__ __noinline__ int rkf_pair(double eps_th, double xe, double rel
             toldy = fmin(toldy, fabs(tol / f0[i]));
         }
     }
-    double h = (toldy == 1.7976931348623157e308) ? epsmin * xe : fmin(xe / 100.0, pow(toldy, 0.2));
+    double h = (toldy == 1.7976931348623157e308) ? epsmin * xe : fmin(xe / 100.0, fifth_root(toldy));
     double x = 0.0;
     int ier = 10000, n = 0;
     *error = 0.0;
-    for (int iter = 1; iter <= itemax; iter++) {
-        fehl4(eps_th, h, yl0, yln, er, true);
+    bool last = false;  // the step to the end, its size set, is under way
+    for (int iter = 0;;) {
+        if (!last && ++iter > itemax) break;
+        fehl4<kNormal, true>(eps_th, h, yl0, al, yln, er);
         double erret = 0.0;
-        bool bad = false;
+        if (!last) {
+            bool bad = false;
+            if (relerr == 0.0) {  // one tolerance: the largest |er| over it, one division for four
+                const double m = fmax(fmax(fabs(er[0]), fabs(er[1])), fmax(fabs(er[2]), fabs(er[3])));
+                bad = abserr == 0.0;
+                erret = fmax(0.0, m / abserr);
+            } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const double et = relerr / 2.0 * (fabs(yl0[i]) + fabs(yln[i])) + abserr;
-            if (et == 0.0) bad = true;
-            erret = fmax(erret, fabs(er[i]) / et);
+                for (int i = 0; i < 4; i++) {
+                    const double et = relerr / 2.0 * (fabs(yl0[i]) + fabs(yln[i])) + abserr;
+                    if (et == 0.0) bad = true;
+                    erret = fmax(erret, fabs(er[i]) / et);
+                }
+            }
+            if (bad) { ier = 20000; break; }
+            if (erret > 1.0) {
+                h = (erret >= 59049.0) ? 0.1 * h : 0.9 * h / fifth_root(erret);
+                if (h <= epsmin) { ier = 30000; break; }
+                continue;
+            }
+            if (!(x + h < xe)) {  // the same low step once more, to xe exactly
+                last = true;
+                h = xe - x;
+                continue;
+            }
         }
-        if (bad) { ier = 20000; break; }
-        if (erret > 1.0) {
-            h = (erret >= 59049.0) ? 0.1 * h : 0.9 * h / pow(erret, 0.2);
-            if (h <= epsmin) { ier = 30000; break; }
-        } else if (x + h < xe) {
-            fehl4(eps_th, h * 0.5, yh0, ymid, er, false);
-            fehl4(eps_th, h * 0.5, ymid, yhn, er, false);
-            x = x + h;
+        double ymid[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) { yl0[i] = yln[i]; yh0[i] = yhn[i]; }
-            n++;
-            h = (erret <= 1.889568e-4) ? 5.0 * h : 0.9 * h / pow(erret, 0.2);
-        } else {
-            h = xe - x;
-            fehl4(eps_th, h, yl0, yln, er, true);
-            fehl4(eps_th, h * 0.5, yh0, ymid, er, false);
-            fehl4(eps_th, h * 0.5, ymid, yhn, er, false);
+        for (int i = 0; i < 4; i++) ymid[i] = yh0[i];
+#pragma unroll 1
+        for (int half = 0; half < 2; half++) {
+            double am[2];
+            moon_acc<kNormal>(eps_th, ymid[0], ymid[1], am[0], am[1]);
+            fehl4<kNormal, false>(eps_th, h * 0.5, ymid, am, yhn, er);
+#pragma unroll
+            for (int i = 0; i < 4; i++) ymid[i] = yhn[i];
+        }
+        n++;
+        if (last) {
             double m = (yln[0] - yhn[0]) / 31.0;
 #pragma unroll
             for (int i = 1; i < 4; i++) m = fmax(m, (yln[i] - yhn[i]) / 31.0);
             *error = m;
-            n++;
             ier = 0;
             break;
         }
+        x = x + h;
+#pragma unroll
+        for (int i = 0; i < 4; i++) { yl0[i] = yln[i]; yh0[i] = yhn[i]; }
+        moon_acc<kNormal>(eps_th, yl0[0], yl0[1], al[0], al[1]);
+        h = (erret <= 1.889568e-4) ? 5.0 * h : 0.9 * h / fifth_root(erret);
     }
 #pragma unroll
     for (int i = 0; i < 4; i++) YN[i] = yhn[i];
     *nacc = n;
     return ier;
+}
+
+// The reciprocal-square-root form where the initial separation and its change over the step are far from the
+// ends of the type's range (nothing physical is not), else the reference's divisions.
+__device__ __forceinline__ int rkf_pair(double eps_th, double xe, double relerr, double abserr, const double YZ[4],
+                                        double YN[4], double *error, int *nacc)
+{
+    const double r2 = YZ[0] * YZ[0] + YZ[1] * YZ[1];
+    const double d2 = (YZ[2] * YZ[2] + YZ[3] * YZ[3]) * (xe * xe);
+    if (r2 > 1e-200 && r2 < 1e200 && d2 < 1e200)
+        return rkf_pair_form<true>(eps_th, xe, relerr, abserr, YZ, YN, error, nacc);
+    return rkf_pair_form<false>(eps_th, xe, relerr, abserr, YZ, YN, error, nacc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1085,17 +1203,6 @@ struct UvFastStep {
 __device__ __forceinline__ UvFastStep uv_fast_step(double dt)
 {
     return {dt, dt * dt, dt > 1e-100 && dt < 1e100};
-}
-
-// 1/sqrt(x) of a normal x: the hardware approximation (relative error below 2^-19) and one step
-// of Householder's third-order iteration y (1 + e/2 + 3/8 e^2), e = 1 - x y^2.  Zero, subnormal
-// and infinite x give NaN or infinity, which uv_fast_pair's test turns away.
-__device__ __forceinline__ double rsqrt_normal(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-__dmul_rn(x, y), y, 1.0);
-    return fma(fma(e, 0.375, 0.5), __dmul_rn(y, e), y);
 }
 
 // cdt2: eps_ij dt^2

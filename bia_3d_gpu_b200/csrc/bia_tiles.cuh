@@ -22,7 +22,7 @@ namespace bia {
 #ifndef BIA_ALG_MIN_BLOCKS
 #define BIA_ALG_MIN_BLOCKS 3
 #endif
-// RKF45: the shared-memory column walk at two CTAs per SM (128 registers; 600 B of spills
+// RKF45: the shared-memory column walk at two CTAs per SM (128 registers; 270 B of spills
 // around the out-of-line pair integrator) measured 184 ms per Coulomb step at n = 32768
 // against 245 ms for the shuffle walk at one CTA per SM (222 registers) and 194 ms for the
 // shuffle walk at two; bitwise the same sums.
