@@ -178,6 +178,7 @@ constexpr int kDimCoopMaxBlocks = 1024;  // partials of the cooperative solver's
 // and 6 x 6n for k1..k6; plus reduction scratch and the step size.
 struct DimBuffers {
     double *yl0, *yln, *yh0, *yhm, *yhn, *er, *w, *wb, *k, *red, *h, *scal, *io;
+    double *pos;  // the resident kernel's stage positions, [2 tracks][2 parities][3][n rounded up to even]: over k
 };
 
 struct DimRun {
@@ -333,6 +334,8 @@ static void dim_carve(double *base, int n, DimBuffers &B)
     B.er = base + 5 * len;
     B.w = base + 6 * len;
     B.k = base + 7 * len;
+    // 16-byte aligned (base is, 7 len is even); 12 (n + 1) <= 36 n doubles
+    B.pos = B.k;
     B.wb = base + 13 * len;
     B.red = base + 14 * len;
     B.h = B.red + kDimCoopMaxBlocks;
@@ -370,8 +373,8 @@ struct DimCoopArgs {
 // shared memory (coalesced structure-of-arrays loads, one element per thread and
 // component); thread (particle lane, chunk c) of the block's P x C threads (C = 256 / P)
 // adds the tile's entries c, c + C, ..., and the C chunk sums of a particle are added in
-// chunk order at the end (deterministic).  P = 8 below n = 4096 (more groups than SMs at
-// small n), 32 above (each tile then serves 32 particles, 32 entries per thread).
+// chunk order at the end (deterministic).  P = 32: each tile serves 32 particles, 32 entries per
+// thread.  It takes the sizes beyond the resident kernel below (about 35000 particles on 148 SMs).
 //
 // Inverse cube: kFastInv (bia_dim_integrate) eps r^-3 from one rsqrt (r^-1, then its cube;
 // rsqrt is within 1 ulp, the product within ~4 ulp of eps / r^3); otherwise the
@@ -626,6 +629,481 @@ __global__ void __launch_bounds__(256) dim_coop_kernel(const DimCoopArgs A)
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// The resident solver: the same integration with every particle's whole state (tracks, stage derivatives)
+// in the shared memory of the CTA that owns it, one CTA per SM.  Between stages only the stage
+// positions cross the device: a CTA publishes its particles' (24 bytes each), the grid meets, and
+// every CTA streams all positions through shared memory in double-buffered tiles.
+//
+// A derivative of dim_coop_kernel took 6 us at n = 200 and 12 at 1332, mostly latency: stage sums through
+// global memory, 8 warps per SM on the forces, a serial loop over the blocks' error norms.  Here
+// * 16 warps share a CTA's particles: lanes hold P x R of them (R in registers, P across lanes) and the
+//   32/P lane groups of the 16 warps split the tile's positions (dim_shape picks P and R);
+// * the low track's step and the high track's first half step do not depend on one another and run their
+//   stages together while a stage is mostly latency (dual): 12 grid-wide barriers a step instead of
+//   18.  An attempt that is rejected has done the half step for nothing (rejections are rare);
+// * the error norm's partials travel with the last stage and are read by one warp;
+// * the integration is one loop over stages, so that nothing lives in local memory across a barrier (its
+//   fence empties L1).
+// Forces: eps r^-3 by the reciprocal square root's approximation and one third-order step, 15 FP64
+// operations an interaction (the sum takes eps once); a particle whose sum is not finite (positions
+// beyond 1e154) is summed again with rsqrt.
+//
+// Measured, a derivative: n = 200 3.1 us (dim_coop_kernel 6.0), 1332 7.4 (11.9), 4096 26 (56), 6000 54 (97), 32768
+// 1183 (2204).  What bounds it: at n = 32768 the interactions (35 cycles of register reads each, 85 % of
+// the stage); at 1332 they are 9200 of a stage's 21000 cycles, the barrier 3600, fetching the
+// positions 3400, the sums 3300; at 200 latency throughout.
+constexpr int kResThreads = 512;
+constexpr int kResWarps = kResThreads / 32;
+constexpr int kResMaxR = 7;
+
+struct DimResArgs {
+    int n, npad, own;  // own: particles per CTA (the last may have fewer)
+    int P, init, itemax;
+    int dual;          // low step and first half step together
+    int tile;          // positions per tile
+    int rows;          // rows of warp sums kept at a time: 16, 8 or 4
+    double eps, relerr, abserr, xe;
+    double *pos;  // [2 tracks][2 parities][3][npad]
+    double *red;  // [gridDim.x]
+    double *y, *ese, *yl0, *er, *io;  // as DimCoopArgs
+};
+
+// shared memory, in doubles: two tiles, the warps' partial sums, the forces of two tracks, their stage velocities
+// (two parities), five state vectors, the error, the stage derivatives of one or two tracks
+static size_t res_smem_doubles(int own, int slots, int tile, int rows, bool dual)
+{
+    return 2 * 3 * (size_t)tile + (size_t)rows * 3 * slots + (6 + 12 + 36 + (dual ? 72 : 36)) * (size_t)own;
+}
+
+__device__ __forceinline__ void cp_async16(double *dst, const double *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// force on a particle whose sum overflowed: every position again, rsqrt's full range
+static __device__ __noinline__ double dim_force_again(const double *pos, int n, int npad, int i, int c, double eps)
+{
+    const double xi = __ldcg(pos + i), yi = __ldcg(pos + npad + i), zi = __ldcg(pos + 2 * (size_t)npad + i);
+    double a = 0.0;
+    for (int j = 0; j < n; j++) {
+        const double d[3] = {xi - __ldcg(pos + j), yi - __ldcg(pos + npad + j), zi - __ldcg(pos + 2 * (size_t)npad + j)};
+        const double rsq = d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + 1e-99;
+        const double ir = rsqrt(rsq);
+        a += d[c] * (eps * (ir * ir * ir));
+    }
+    return a;
+}
+
+// maximum (negative wins) or minimum
+__device__ __forceinline__ double res_pick(double a, double b, bool take_max)
+{
+    return take_max ? ((a < 0.0 || b < 0.0) ? -1.0e300 : fmax(a, b)) : fmin(a, b);
+}
+
+extern __shared__ __align__(16) double res_smem[];
+
+// What a pass over six stages is: the first step size, an attempted low step (with the first half step when
+// dual), the half steps of an accepted one, and the same to the end.
+enum ResPhase { kResInit, kResTry, kResHalf1, kResHalf2, kResLast, kResLastHalf1, kResLastHalf2, kResDone };
+
+template <int R, bool kFastInv>
+__global__ void __launch_bounds__(kResThreads, 1) dim_resident_kernel(const DimResArgs A)
+{
+    cg::grid_group grid = cg::this_grid();
+    __shared__ double s_red[kResWarps];
+    __shared__ double s_total;
+    const double EPSMIN = 1e-15;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int own = A.own, P = A.P, slots = P * R, npad = A.npad;
+    const int first = blockIdx.x * own, mine = min(own, A.n - first);
+    const int ntiles = (A.n + A.tile - 1) / A.tile;
+    double *const tiles = res_smem;                 // [2][3][tile]
+    double *const part = tiles + 2 * 3 * A.tile;    // [rows][3][slots]
+    double *const force = part + A.rows * 3 * slots;  // [2][3][own]
+    double *const vel = force + 6 * own;            // [2 tracks][2 stage parities][3][own]
+    double *const vec = vel + 12 * own;             // the state vectors, [6][own] each
+    const int vlen = 6 * own;
+    double *yl0 = vec, *yln = vec + vlen, *yh0 = vec + 2 * vlen, *yhn = vec + 3 * vlen;
+    double *const yhm = vec + 4 * vlen, *const er = vec + 5 * vlen;
+    double *const kbuf = vec + 6 * vlen;            // [1 or 2][6 stages][6][own]
+    const size_t track = 6 * (size_t)npad, half = 3 * (size_t)npad;
+
+    // positions of state vector y as track t's next stage input
+    auto publish = [&](int t, const double *y, int parity) {
+        double *dst = A.pos + t * track + parity * half + first;
+        for (int e = tid; e < 96; e += kResThreads) {  // three warps, one a component
+            for (int i = lane; i < mine; i += 32) dst[(size_t)warp * npad + i] = y[warp * own + i];
+        }
+    };
+    // the block's value over its threads' v, into its slot of A.red, before a barrier
+    auto block_value = [&](double v, bool take_max) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = res_pick(v, __shfl_xor_sync(0xffffffffu, v, o), take_max);
+        if (lane == 0) s_red[warp] = v;
+        __syncthreads();
+        if (tid == 0) {
+            double m = s_red[0];
+            for (int w = 1; w < kResWarps; w++) m = res_pick(m, s_red[w], take_max);
+            A.red[blockIdx.x] = m;
+        }
+    };
+    // the grid's value, after the barrier: every CTA reads the same partials
+    auto grid_value = [&](bool take_max) {
+        if (warp == 0) {
+            double m = take_max ? 0.0 : INFINITY;
+            for (int b = lane; b < (int)gridDim.x; b += 32) m = res_pick(m, __ldcg(A.red + b), take_max);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = res_pick(m, __shfl_xor_sync(0xffffffffu, m, o), take_max);
+            if (lane == 0) s_total = m;
+        }
+        __syncthreads();
+        return s_total;
+    };
+
+    for (int c = warp; c < 6; c += kResWarps)
+        for (int i = lane; i < mine; i += 32)
+            yl0[c * own + i] = yh0[c * own + i] = A.y[(size_t)c * A.n + first + i];
+    double X = A.io[0], H = A.io[1];
+    int nde = 0, acc = 0, rej = 0, iter = 0, ier = 10000, parity = 0, s = 0;
+    int phase = A.init == 1 ? kResInit : kResTry;
+    bool to_end = false;  // the attempted step reaches xe
+    __syncthreads();
+    publish(0, yl0, parity);
+    publish(1, yh0, parity);
+    grid.sync();
+    if (phase == kResTry) to_end = !(X + H < A.xe);
+
+#pragma unroll 1
+    while (phase != kResDone) {
+        // the tracks of this stage: t0 .. t0 + nt - 1, from y0 by h into yn
+        const int t0 = (phase == kResHalf1 || phase == kResHalf2 || phase == kResLastHalf1 || phase == kResLastHalf2) ? 1 : 0;
+        const int nt = (A.dual && ((phase == kResTry && !to_end) || phase == kResLast)) ? 2 : 1;
+
+        // forces of this CTA's particles in those tracks from their published positions
+        {
+            const int total = nt * ntiles;
+            const double *src0 = A.pos + t0 * track + parity * half;
+            auto issue = [&](int q) {
+                const int u = q >= ntiles ? 1 : 0, jt = q - u * ntiles;
+                const double *src = src0 + u * track + jt * A.tile;
+                double *dst = tiles + (q & 1) * 3 * A.tile;
+                const int pieces = (min(A.tile, A.n - jt * A.tile) + 1) / 2;  // 16 bytes (npad is even)
+                for (int e = tid; e < pieces; e += kResThreads) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++) cp_async16(dst + c * A.tile + 2 * e, src + (size_t)c * npad + 2 * e);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+            issue(0);
+            if (total > 1) issue(1);
+            const int pi = lane & (P - 1);
+            const int js = lane / P + (32 / P) * warp, nj = kResThreads / P;
+            double xi[R], yi[R], zi[R], ax[R], ay[R], az[R];
+#pragma unroll 1
+            for (int q = 0; q < total; q++) {
+                const int u = q >= ntiles ? 1 : 0, jt = q - u * ntiles;
+                if (jt == 0) {
+                    const double *p = src0 + u * track;
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const int i = min(first + min(r * P + pi, own - 1), A.n - 1);
+                        xi[r] = __ldcg(p + i);
+                        yi[r] = __ldcg(p + npad + i);
+                        zi[r] = __ldcg(p + 2 * (size_t)npad + i);
+                        ax[r] = ay[r] = az[r] = 0.0;
+                    }
+                }
+                if (q + 1 < total) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncthreads();
+                const double *T = tiles + (q & 1) * 3 * A.tile;
+                const int cnt = min(A.tile, A.n - jt * A.tile);
+                constexpr int kUnroll = R >= 3 ? 1 : R == 2 ? 2 : 4;  // chains side by side; more spills
+#pragma unroll kUnroll
+                for (int j = js; j < cnt; j += nj) {
+                    const double xj = T[j], yj = T[A.tile + j], zj = T[2 * A.tile + j];
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        const double dx = xi[r] - xj, dy = yi[r] - yj, dz = zi[r] - zj;
+                        if (kFastInv) {
+                            const double rsq = fma(dx, dx, fma(dy, dy, fma(dz, dz, 1e-99)));
+                            double y;
+                            asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(rsq));
+                            const double y2 = y * y;  // exact: the low half of y is zero
+                            const double e = fma(-rsq, y2, 1.0);
+                            const double y3 = y * y2;
+                            const double w = fma(y3 * e, fma(e, 1.875, 1.5), y3);
+                            ax[r] = fma(dx, w, ax[r]);
+                            ay[r] = fma(dy, w, ay[r]);
+                            az[r] = fma(dz, w, az[r]);
+                        } else {
+                            const double rsq = dx * dx + dy * dy + dz * dz + 1e-99;
+                            const double w = A.eps / (rsq * sqrt(rsq));
+                            ax[r] += dx * w;
+                            ay[r] += dy * w;
+                            az[r] += dz * w;
+                        }
+                    }
+                }
+                if (jt == ntiles - 1) {
+                    // the lane groups' sums, the warps' onto A.rows rows in turn, then the rows in order
+                    for (int o = P; o < 32; o <<= 1) {
+#pragma unroll
+                        for (int r = 0; r < R; r++) {
+                            ax[r] += __shfl_xor_sync(0xffffffffu, ax[r], o);
+                            ay[r] += __shfl_xor_sync(0xffffffffu, ay[r], o);
+                            az[r] += __shfl_xor_sync(0xffffffffu, az[r], o);
+                        }
+                    }
+                    double *pw = part + (warp & (A.rows - 1)) * 3 * slots;
+                    for (int w0 = 0; w0 < kResWarps; w0 += A.rows) {
+                        if (warp >= w0 && warp < w0 + A.rows && lane < P) {
+#pragma unroll
+                            for (int r = 0; r < R; r++) {
+                                const int sl = r * P + lane;
+                                pw[sl] = (w0 == 0 ? 0.0 : pw[sl]) + ax[r];
+                                pw[slots + sl] = (w0 == 0 ? 0.0 : pw[slots + sl]) + ay[r];
+                                pw[2 * slots + sl] = (w0 == 0 ? 0.0 : pw[2 * slots + sl]) + az[r];
+                            }
+                        }
+                        __syncthreads();
+                    }
+                    // one lane a row, two sums a warp (rows beyond A.rows add zero)
+                    for (int e = 2 * warp + (lane >> 4); e - (lane >> 4) < 3 * mine; e += 2 * kResWarps) {
+                        const int c = e < mine ? 0 : e < 2 * mine ? 1 : 2, i = e - c * mine, w = lane & 15;
+                        double a = e < 3 * mine && w < A.rows ? part[(w * 3 + c) * slots + i] : 0.0;
+#pragma unroll
+                        for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                        if (w == 0 && e < 3 * mine) {
+                            if (kFastInv) {
+                                a *= A.eps;
+                                if (!isfinite(a)) a = dim_force_again(src0 + u * track, A.n, npad, first + i, c, A.eps);
+                            }
+                            force[((t0 + u) * 3 + c) * own + i] = a;
+                        }
+                    }
+                }
+                __syncthreads();  // the tile's buffer is free; the forces are there
+                if (q + 2 < total) issue(q + 2);
+            }
+        }
+
+        if (phase == kResInit) {  // first step size (dim/rkf_kernel.cu:248-261)
+            double m = INFINITY;
+            for (int c = warp; c < 6; c += kResWarps)
+                for (int i = lane; i < mine; i += 32) {
+                    const double k1 = c < 3 ? yl0[(3 + c) * own + i] : force[(c - 3) * own + i];
+                    if (fabs(k1) > 0.0) m = fmin(m, fabs((A.relerr * fabs(yl0[c * own + i]) + A.abserr) / k1));
+                }
+            block_value(m, false);
+            grid.sync();
+            const double toldy = grid_value(false);
+            H = isinf(toldy) ? EPSMIN * (A.xe - X) : fmin((A.xe - X) / 100e0, pow(toldy, 0.2));
+            nde = 1;
+            phase = kResTry;
+            to_end = !(X + H < A.xe);
+            continue;
+        }
+
+        // stage s of those tracks: its derivative, and the next stage's input or, after the sixth, the new state
+        double worst = 0.0;
+        for (int row = warp; row < 6 * nt; row += kResWarps) {
+            const int t = t0 + (row >= 6 ? 1 : 0), c = row >= 6 ? row - 6 : row;
+            const double *y0 = t == 0 ? yl0 : (phase == kResHalf2 || phase == kResLastHalf2) ? yhm : yh0;
+            double *yn = t == 0 ? yln : (phase == kResHalf2 || phase == kResLastHalf2) ? yhn : yhm;
+            const double h = t == 0 ? H : H / 2;
+            double *k0 = kbuf + (A.dual ? t : 0) * 6 * vlen + c * own;  // stage m at m vlen
+            double *v = vel + t * vlen;                                  // [2 stage parities][3][own]
+            for (int i = lane; i < mine; i += 32) {
+                double *k = k0 + i;
+                k[s * vlen] = c >= 3 ? force[(t * 3 + c - 3) * own + i]
+                            : s == 0 ? y0[(3 + c) * own + i]
+                                     : v[((s & 1) * 3 + c) * own + i];
+                double sum = 0.0;
+                if (s == 0) {
+                    sum = h * c_fehl[0][0] * k[0];
+                } else {
+                    for (int m = 0; m <= s; m++) sum += c_fehl[s][m] * k[m * vlen];
+                    sum = h * sum;
+                }
+                const double y = y0[c * own + i], w = y + sum;
+                if (s < 5) {
+                    if (c < 3) A.pos[t * track + (parity ^ 1) * half + (size_t)c * npad + first + i] = w;
+                    else v[(((s + 1) & 1) * 3 + c - 3) * own + i] = w;
+                } else {
+                    yn[c * own + i] = w;
+                    if (t == 0) {
+                        double ae = 0.0;
+                        for (int m = 0; m < 6; m++) ae += c_fehl[6][m] * k[m * vlen];
+                        ae = h * ae;
+                        er[c * own + i] = ae;
+                        const double et = A.relerr * (fabs(y) + fabs(w)) / 2 + A.abserr;
+                        if (et == 0.0) worst = -1.0e300;
+                        else if (worst >= 0.0) worst = fmax(worst, fabs(ae) / et);
+                    }
+                }
+            }
+        }
+        if (s < 5) {
+            grid.sync();
+            parity ^= 1;
+            s++;
+            continue;
+        }
+
+        // after the sixth stage: publish what comes next, meet, decide
+        s = 0;
+        if (phase == kResTry) block_value(worst, true);
+        __syncthreads();
+        if (phase == kResTry || phase == kResLast) {
+            publish(1, nt == 2 ? yhm : yh0, parity ^ 1);
+        } else if (phase == kResHalf1 || phase == kResLastHalf1) {
+            publish(1, yhm, parity ^ 1);
+        } else {
+            publish(0, yln, parity ^ 1);
+            publish(1, yhn, parity ^ 1);
+        }
+        grid.sync();
+        parity ^= 1;
+        if (phase == kResTry) {
+            nde += 6;
+            const double erret = grid_value(true);
+            if (erret < 0.0) {
+                ier = 20000;
+                phase = kResDone;
+            } else if (erret > 1) {
+                rej++;
+                if (erret >= 59049) H *= 0.1;
+                else H *= 0.9 / pow(erret, 0.2);
+                if (H <= EPSMIN) {
+                    ier = 30000;
+                    phase = kResDone;
+                } else if (++iter >= A.itemax) {
+                    phase = kResDone;
+                } else {
+                    publish(0, yl0, parity);
+                    publish(1, yh0, parity);
+                    grid.sync();
+                    to_end = !(X + H < A.xe);
+                }
+            } else if (!to_end) {
+                // the half steps of the high track (fhstep, dim/rkf_kernel.cu:318-362), and the next step's size
+                if (tid == 0) s_red[0] = erret;  // for the end of the second half step
+                phase = nt == 2 ? kResHalf2 : kResHalf1;
+            } else {
+                // last step to xe (dim/rkf_kernel.cu:386-483)
+                H = A.xe - X;
+                publish(0, yl0, parity);
+                publish(1, yh0, parity);
+                grid.sync();
+                phase = kResLast;
+            }
+        } else if (phase == kResHalf1) {
+            phase = kResHalf2;
+        } else if (phase == kResHalf2) {
+            const double erret = s_red[0];
+            nde += 12;
+            X += H;
+            double *t1 = yl0; yl0 = yln; yln = t1;  // accepted: the new tracks become the old ones
+            double *t2 = yh0; yh0 = yhn; yhn = t2;
+            acc++;
+            if (erret <= 1.889568e-4) H *= 5.0;
+            else H *= 0.9 / pow(erret, 0.2);
+            to_end = !(X + H < A.xe);
+            phase = ++iter >= A.itemax ? kResDone : kResTry;
+        } else if (phase == kResLast) {
+            phase = nt == 2 ? kResLastHalf2 : kResLastHalf1;
+        } else if (phase == kResLastHalf1) {
+            phase = kResLastHalf2;
+        } else {
+            nde += 18;
+            X = A.xe;
+            acc++;
+            ier = 0;
+            phase = kResDone;
+        }
+    }
+    __syncthreads();
+    // outputs as dim_coop_kernel's: the state (the high track at xe, or the last accepted one), the low track,
+    // (yln - yhn) / 31 and the last error estimate
+    const double *yout = (ier == 0) ? yhn : yh0, *lout = (ier == 0) ? yln : yl0;
+    for (int c = warp; c < 6; c += kResWarps)
+        for (int i = lane; i < mine; i += 32) {
+            const int at = c * own + i;
+            const size_t g = (size_t)c * A.n + first + i;
+            if (A.ese && ier == 0) A.ese[g] = (yln[at] - yhn[at]) / 31;
+            A.y[g] = yout[at];
+            A.yl0[g] = lout[at];
+            A.er[g] = er[at];
+        }
+    if (blockIdx.x == 0 && tid == 0) {
+        A.io[0] = X;
+        A.io[1] = H;
+        A.io[2] = nde;
+        A.io[3] = (double)acc;
+        A.io[4] = (double)rej;
+        A.io[5] = ier;
+    }
+}
+
+// Slots of the resident kernel for `own` particles per CTA: P across lanes, R in registers, the cheapest in
+// cycles of the SM: 35 register-port cycles an interaction and warp on four schedulers and 12 a position
+// read, and 64 for each value and step of the lane groups' sums (two shuffles from each of 16 warps, two
+// cycles each).  Measured at n = 1332: P, R = 4, 3 11000 cycles a stage, 16, 1 12500.
+static void dim_shape(int n, int own, int *P, int *R)
+{
+    double best = 0.0;
+    *P = *R = 0;
+    for (int p = 1, lg = 5; p <= 32; p *= 2, lg--) {
+        const int r = (own + p - 1) / p;
+        if (r > kResMaxR) continue;
+        const double per_warp = (double)r * (double)((n + kResThreads / p - 1) / (kResThreads / p));
+        const double cost = (140.0 + 48.0 / r) * per_warp + 192.0 * r * lg;
+        if (*R == 0 || cost < best) {
+            best = cost;
+            *P = p;
+            *R = r;
+        }
+    }
+}
+
+template <bool kFastInv>
+static const void *dim_resident_form(int R)
+{
+    switch (R) {
+    case 1: return (const void *)dim_resident_kernel<1, kFastInv>;
+    case 2: return (const void *)dim_resident_kernel<2, kFastInv>;
+    case 3: return (const void *)dim_resident_kernel<3, kFastInv>;
+    case 4: return (const void *)dim_resident_kernel<4, kFastInv>;
+    case 5: return (const void *)dim_resident_kernel<5, kFastInv>;
+    case 6: return (const void *)dim_resident_kernel<6, kFastInv>;
+    default: return (const void *)dim_resident_kernel<7, kFastInv>;
+    }
+}
+
+// The resident kernel's launch for n particles on a device with `sms` SMs: false where the particles do not fit
+// (more than kResMaxR x 32 a CTA, or the shared memory).  Larger tiles, more rows of warp sums and both
+// tracks at once as far as the shared memory goes; both tracks only while a stage is mostly latency
+// (measured at n = 6000 either way the same).
+static bool dim_resident_plan(int n, int sms, size_t max_smem, DimResArgs &A, int *G, int *R, size_t *bytes)
+{
+    A.own = (n + sms - 1) / sms;
+    *G = (n + A.own - 1) / A.own;
+    if (*G > kDimCoopMaxBlocks) return false;
+    dim_shape(n, A.own, &A.P, R);
+    if (*R == 0) return false;
+    for (int level = n <= 4096 ? 0 : 1; level < 4; level++) {
+        A.dual = level == 0;
+        A.tile = level < 3 ? 1024 : 512;
+        A.rows = level < 2 ? kResWarps : 4;
+        *bytes = res_smem_doubles(A.own, A.P * *R, A.tile, A.rows, A.dual != 0) * sizeof(double);
+        if (*bytes <= max_smem) return true;
+    }
+    return false;
+}
+
 // The cooperative solver (dim_coop_kernel); *ran = false when the device cannot run it
 // (no cooperative launch), and the caller takes the host-controlled loop instead.
 static int dim_integrate_coop(DimRun &R, double *y, double *x0, double xe, int init, double *H, int *nde,
@@ -639,41 +1117,70 @@ static int dim_integrate_coop(DimRun &R, double *y, double *x0, double xe, int i
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    // groups of 8 particles below n = 4096, of 32 above; the inverse-cube form of the run
-    const bool wide = R.n >= 4096;
-    const void *kern = wide ? (R.fast_inv ? (const void *)dim_coop_kernel<32, true> : (const void *)dim_coop_kernel<32, false>)
-                            : (R.fast_inv ? (const void *)dim_coop_kernel<8, true> : (const void *)dim_coop_kernel<8, false>);
-    const int P = wide ? 32 : 8;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        return 0;
-    }
-    const int ngroups = (R.n + P - 1) / P;
-    int G = ngroups;
-    if (G > sms * per_sm) G = sms * per_sm;
-    if (G > kDimCoopMaxBlocks) G = kDimCoopMaxBlocks;  // B.red holds kDimCoopMaxBlocks partials
-    const char *gcap = getenv("BIA_DIM_COOP_BLOCKS");
-    if (gcap && atoi(gcap) > 0 && atoi(gcap) < G) G = atoi(gcap);
-    if (G < 1) G = 1;
-    DimCoopArgs A;
-    A.n = R.n;
-    A.len = R.len;
-    A.init = init;
-    A.itemax = 10000;
-    A.eps = R.eps;
-    A.relerr = R.relerr;
-    A.abserr = R.abserr;
-    A.xe = xe;
-    A.B = R.B;
-    A.y = y;
-    A.ese = ese;
-    A.io = R.B.io;
+    int max_smem = 0;
+    if (cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    max_smem -= 1024;  // the kernel's static shared memory
     R.h_pinned[0] = *x0;
     R.h_pinned[1] = *H;
+    int G = 0, reg = 0;
+    size_t bytes = 0;
+    const void *kern = nullptr;
+    DimResArgs B;
+    DimCoopArgs A;
+    void *args[1];
+    const char *gcap = getenv("BIA_DIM_COOP_BLOCKS");  // a cap on the blocks: the global-memory kernel's
+    const int cap = gcap ? atoi(gcap) : 0;
+    if (cap <= 0 && dim_resident_plan(R.n, sms, (size_t)max_smem, B, &G, &reg, &bytes)) {
+        kern = R.fast_inv ? dim_resident_form<true>(reg) : dim_resident_form<false>(reg);
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        B.n = R.n;
+        B.npad = (R.n + 1) & ~1;
+        B.init = init;
+        B.itemax = 10000;
+        B.eps = R.eps;
+        B.relerr = R.relerr;
+        B.abserr = R.abserr;
+        B.xe = xe;
+        B.pos = R.B.pos;
+        B.red = R.B.red;
+        B.y = y;
+        B.ese = ese;
+        B.yl0 = R.B.yl0;
+        B.er = R.B.er;
+        B.io = R.B.io;
+        args[0] = (void *)&B;
+    } else {
+        // too many particles for the SMs' shared memory: groups of 32, all state in global memory
+        kern = R.fast_inv ? (const void *)dim_coop_kernel<32, true> : (const void *)dim_coop_kernel<32, false>;
+        bytes = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1) {
+            cudaGetLastError();
+            return 0;
+        }
+        G = (R.n + 31) / 32;
+        if (G > sms * per_sm) G = sms * per_sm;
+        if (G > kDimCoopMaxBlocks) G = kDimCoopMaxBlocks;  // B.red holds kDimCoopMaxBlocks partials
+        if (cap > 0 && cap < G) G = cap;
+        A.n = R.n;
+        A.len = R.len;
+        A.init = init;
+        A.itemax = 10000;
+        A.eps = R.eps;
+        A.relerr = R.relerr;
+        A.abserr = R.abserr;
+        A.xe = xe;
+        A.B = R.B;
+        A.y = y;
+        A.ese = ese;
+        A.io = R.B.io;
+        args[0] = (void *)&A;
+    }
     cudaError_t e = cudaMemcpyAsync(R.B.io, R.h_pinned, 2 * sizeof(double), cudaMemcpyHostToDevice, R.st);
-    void *args[] = {(void *)&A};
     if (e == cudaSuccess)
-        e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(256), args, 0, R.st);
+        e = cudaLaunchCooperativeKernel(kern, dim3(G), dim3(bytes ? kResThreads : 256), args, bytes, R.st);
     double out[6] = {0, 0, 0, 0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(R.h_pinned, R.B.io, 6 * sizeof(double), cudaMemcpyDeviceToHost, R.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(R.st);
