@@ -22,36 +22,6 @@ namespace bia {
 
 constexpr double kPi = 3.14159265358979323846264338327950288419716939937510582097494;
 
-// Optional out-of-line FP64 math: each libm call site expands to a long instruction
-// sequence; routing the calls through one copy shrinks the code.  Measured on B200
-// (n = 32768, 3 CTAs/SM): out-of-line math and hyp_eval 204 ms (Coulomb, mixed orbit
-// classes) / 88 ms (Plummer, hyperbolae only) per step, everything inline 213 / 73 ms;
-// inline is the default.
-#ifndef BIA_NOINLINE_MATH
-#define BIA_NOINLINE_MATH 0
-#endif
-#if BIA_NOINLINE_MATH
-static __device__ __noinline__ void d_sincos(double x, double *s, double *c) { sincos(x, s, c); }
-static __device__ __noinline__ double d_log(double x) { return log(x); }
-static __device__ __noinline__ double d_atan2(double y, double x) { return atan2(y, x); }
-static __device__ __noinline__ double d_acos(double x) { return acos(x); }
-static __device__ __noinline__ double d_atan(double x) { return atan(x); }
-#else
-__device__ __forceinline__ void d_sincos(double x, double *s, double *c) { sincos(x, s, c); }
-__device__ __forceinline__ double d_log(double x) { return log(x); }
-__device__ __forceinline__ double d_atan2(double y, double x) { return atan2(y, x); }
-__device__ __forceinline__ double d_acos(double x) { return acos(x); }
-__device__ __forceinline__ double d_atan(double x) { return atan(x); }
-#endif
-#ifndef BIA_NOINLINE_HYPEVAL
-#define BIA_NOINLINE_HYPEVAL 0
-#endif
-#if BIA_NOINLINE_HYPEVAL
-#define BIA_HYPEVAL_INLINE static __device__ __noinline__
-#else
-#define BIA_HYPEVAL_INLINE __device__ __forceinline__
-#endif
-
 enum PairClass { kHyperbola = 0, kParabola = 1, kEllipse = 2, kDegenerate = 3, kRkf = 4, kUniversal = 5 };
 
 // |e^2 - 1| below which ALG pairs use the universal-variable solver
@@ -89,20 +59,41 @@ __device__ __forceinline__ void counters_zero(PairCounters &c)
     c.learned = c.learned_fallbacks = c.learned_coarse = c.timeouts = c.learned_fp32 = 0;
 }
 
-#ifndef BIA_DIRECT_HALF_SINES
-#define BIA_DIRECT_HALF_SINES 0
-#endif
-#ifndef BIA_STRICT_SETUP
-#define BIA_STRICT_SETUP 0
-#endif
-#ifndef BIA_REF_END_STATE
-#define BIA_REF_END_STATE 1
-#endif
-// Uncontracted IEEE operations, in the oracle's (the reference's) order: the frame and the
-// hyperbola's start angle acos(cs_0 + b sn_0 / r) are ill-conditioned near pericentre
-// (d theta / d arg ~ 1 / sqrt(1 - arg)), so an ulp of difference in the argument becomes
-// up to ~1e-10 of displacement; these values are formed exactly as the CPU path forms
-// them (no fused multiply-add, divisions instead of reciprocals).
+// 1/sqrt(x) of a normal x: the hardware approximation and one step
+// of Householder's third-order iteration y (1 + e/2 + 3/8 e^2), e = 1 - x y^2 (measured
+// at most 2^-19.04 over 1e9 values; the next term, 5/16 e^3, is below 3e-18).  Zero, subnormal
+// and infinite x give NaN or infinity: its callers test for them.
+__device__ __forceinline__ double rsqrt_normal(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-__dmul_rn(x, y), y, 1.0);
+    return fma(fma(e, 0.375, 0.5), __dmul_rn(y, e), y);
+}
+
+// c x^(-3/2) of a normal x from the same approximation y, whose square is exact (its low half is zero):
+// c y^3 (1 + 3/2 e + 15/8 e^2), e = 1 - x y^2; the next term, 35/16 e^3, is below 3e-17.
+__device__ __forceinline__ double scaled_rsqrt3_normal(double c, double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double y2 = y * y;
+    const double e = fma(-x, y2, 1.0);
+    const double c3 = (c * y) * y2;
+    return fma(c3 * e, fma(e, 1.875, 1.5), c3);
+}
+
+// 1/x of a normal x with a normal reciprocal: the hardware approximation y and one third-order step
+// y (1 + e + e^2), e = 1 - x y (the next term, e^3, is below 1e-17).  Zero gives NaN.
+__device__ __forceinline__ double rcp_normal(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
+// Uncontracted IEEE operations: the frame is formed as the CPU path forms it.
 __device__ __forceinline__ double m_(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double a_(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double s_(double a, double b) { return __dsub_rn(a, b); }
@@ -141,21 +132,13 @@ __device__ __forceinline__ bool frame_xi_eta(const double r[3], const double g[3
         return true;
     }
     double ez[3];
-#if BIA_STRICT_SETUP
-    const double Lm = __dsqrt_rn(Lsq);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        e_eta[k] = d_(g[k], gm);
-        ez[k] = d_(L[k], Lm);
-    }
-#else
-    const double iL = 1.0 / sqrt(Lsq), ig = 1.0 / gm;
+    const double iL = Lsq > 1e-290 ? rsqrt_normal(Lsq) : 1.0 / sqrt(Lsq);
+    const double ig = gsq > 1e-290 ? rsqrt_normal(gsq) : 1.0 / gm;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         e_eta[k] = g[k] * ig;
         ez[k] = L[k] * iL;
     }
-#endif
     e_xi[0] = s_(m_(e_eta[1], ez[2]), m_(e_eta[2], ez[1]));
     e_xi[1] = s_(m_(e_eta[2], ez[0]), m_(e_eta[0], ez[2]));
     e_xi[2] = s_(m_(e_eta[0], ez[1]), m_(e_eta[1], ez[0]));
@@ -176,36 +159,46 @@ __device__ __forceinline__ bool frame_xi_eta(const double r[3], const double g[3
 // so one sincos replaces the reference's sin, sin and sincos per evaluation, and the
 // denominator cos theta - cos theta_0 is a product instead of a difference.
 // ---------------------------------------------------------------------------
+constexpr double kFewUlps = 8.9e-16;  // four ulps of 1
+
 struct HypConsts {
-    double theta_0, tn_0, cs_0, sn_0, s0h, c0h, time_end_;
+    double tn_0, cs_0, sn_0, s0h, c0h, time_end_;
 };
 
-// sin((theta_0 +- theta)/2) from the half angles.  Near theta = +-theta_0 (far along an
-// asymptote) the difference of products cancels, so below 0.25 the sine of the small half
-// angle is taken directly, as the reference computes it (bia/find_hyperbola.f90:157-158).
-__device__ __forceinline__ void half_sines(const HypConsts &c, double theta, double sh, double ch, double &sp,
-                                          double &sm)
+// (sh, ch) of half an angle in (-pi, pi] from its sine and cosine, without cancellation
+__device__ __forceinline__ void half_angle(double sn, double cs, double &sh, double &ch)
 {
-    sp = c.s0h * ch + c.c0h * sh;
-    sm = c.s0h * ch - c.c0h * sh;
-#if BIA_DIRECT_HALF_SINES
-    if (fabs(sm) < 0.25) sm = sin(0.5 * (c.theta_0 - theta));
-    if (fabs(sp) < 0.25) sp = sin(0.5 * (c.theta_0 + theta));
-#endif
+    const double t = fma(0.5, fabs(cs), 0.5);
+    const double it = rsqrt_normal(t);
+    const double big = t * it, small = 0.5 * sn * it;  // cos or sin of the half angle, and the other
+    ch = cs >= 0.0 ? big : fabs(small);
+    sh = cs >= 0.0 ? small : copysign(big, sn);
 }
 
 // find_theta (bia/find_hyperbola.f90:149-165): residual e and derivative d at theta;
-// sp, sm = sin((theta_0 +- theta)/2) for the bracket test.
-BIA_HYPEVAL_INLINE void hyp_eval(const HypConsts &c, double theta, double &e, double &d,
+// sp, sm = sin((theta_0 +- theta)/2) for the bracket test.  kFast: one reciprocal for
+// 1/(2 sp sm) and sp/sm (sp sm inside the bracket, so not zero); else divisions, whose infinities
+// at the bracket's ends hyp_safe needs.
+template <bool kFast = true>
+__device__ __forceinline__ void hyp_eval(const HypConsts &c, double theta, double &e, double &d,
                                          double &sp, double &sm)
 {
     double sh, ch;
-    d_sincos(0.5 * theta, &sh, &ch);
-    half_sines(c, theta, sh, ch, sp, sm);
-    const double Dinv = 1.0 / (2.0 * sp * sm);
+    sincos(0.5 * theta, &sh, &ch);
+    sp = c.s0h * ch + c.c0h * sh;
+    sm = c.s0h * ch - c.c0h * sh;
+    double Dinv, ratio;
+    if (kFast) {
+        const double i = rcp_normal(sp * sm);
+        Dinv = 0.5 * i;
+        ratio = sp * sp * i;
+    } else {
+        Dinv = 1.0 / (2.0 * sp * sm);
+        ratio = sp / sm;
+    }
     const double sn = 2.0 * sh * ch;
     const double cs = 1.0 - 2.0 * sh * sh;
-    e = c.tn_0 * sn * Dinv - c.time_end_ + d_log(sp / sm);
+    e = c.tn_0 * sn * Dinv - c.time_end_ + log(ratio);
     d = c.tn_0 * (1.0 - c.cs_0 * cs) * (Dinv * Dinv) + c.sn_0 * Dinv;
 }
 
@@ -214,12 +207,13 @@ BIA_HYPEVAL_INLINE void hyp_eval(const HypConsts &c, double theta, double &e, do
 // increasing for repulsive pairs (tn_0 > 0), decreasing for attractive ones.
 static __device__ __noinline__ double hyp_safe(const HypConsts c, double x)
 {
-    double lo = -c.theta_0, hi = c.theta_0;
+    const double theta_0 = atan2(c.sn_0, c.cs_0);
+    double lo = -theta_0, hi = theta_0;
     const double dir = (c.tn_0 > 0.0) ? 1.0 : -1.0;
     if (!(x > lo && x < hi)) x = 0.0;
     for (int it = 0; it < 400; it++) {
         double f, d, sp, sm;
-        hyp_eval(c, x, f, d, sp, sm);
+        hyp_eval<false>(c, x, f, d, sp, sm);
         if (f == 0.0) break;
         if (f * dir < 0.0) lo = x; else hi = x;
         double xn = x - f / d;
@@ -230,101 +224,106 @@ static __device__ __noinline__ double hyp_safe(const HypConsts c, double x)
     return x;
 }
 
+// The reference's second candidate start, from the atan guess (bia/find_hyperbola.f90:71-89): its
+// residual there and the start one Newton step on.
+static __device__ __noinline__ double hyp_guess(const HypConsts c, double *error)
+{
+    const double theta_0 = atan2(c.sn_0, c.cs_0);
+    const double theta = 2.0 / kPi * theta_0 * atan(c.time_end_ / c.tn_0);
+    double d, sp, sm;
+    hyp_eval<false>(c, theta, *error, d, sp, sm);
+    return (*error == 0.0) ? theta : theta - *error / d;
+}
+
+// Divisions and roots are reciprocals and reciprocal roots shared between the quantities that need
+// them.  The start's sine and cosine are formed from the state, cos theta = cos theta_0 + b sin theta_0/r
+// and sin theta = +-(r.g/r) sin theta_0/g_0, and its angle from both by atan2, where the reference takes
+// acos of the cosine (an ulp of it near pericentre is up to 1e-10 of displacement) and sines and
+// cosines of the angle back; 2 sp sm = cos theta - cos theta_0 = b sin theta_0/r is known without
+// cancellation.  The reference's second start guess is tried only where the Newton step from the start is
+// not small against the distance to the asymptotes (below 1e-3 of it the step's error is 1e-6, and the
+// guess, an angle from scratch, never the better one).
+//
+// What bounds the ALG kernels: FP64 operations in dependent chains (atan2, log, and a sine, cosine and log an
+// evaluation), 46 % of the FP64 pipe and 68 % of the issue slots at 22 of 32 lanes on mixed classes.  So the
+// work per pair is what counts.  Step at n = 32768, Plummer / Coulomb: 71.0 / 83.0 ms with divisions, roots and
+// angles throughout; 43.5 / 54.7 with shared reciprocals and the start's sines from the state (the
+// ellipse's too); 39.1 / 57.0 from the Taylor start, but with the rounding floor still walked by a few
+// lanes; 29.7 / 43.6 when a step of a few ulps ends the iteration (3.1 -> 1.0 evaluations a pair).  The
+// interaction part's error against the exact step went from 8.8e-5 to 6.0e-5 of its norm on Plummer, from 4.0e-8
+// to 3.5e-8 on Coulomb.
 __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, const double YZ[4],
                                          double YN[4], double *error_end, int *bracket_exit,
                                          int *fallback)
 {
     const double X_ini = YZ[0], Y_ini = YZ[1], U_ini = YZ[2], V_ini = YZ[3];
-#if BIA_STRICT_SETUP
-    // up to the start angle: the oracle's operations and order (see m_ above)
-    const double r_g = a_(m_(X_ini, U_ini), m_(Y_ini, V_ini));
-    const double Lz = s_(m_(X_ini, V_ini), m_(Y_ini, U_ini));
-    const double r = __dsqrt_rn(a_(m_(X_ini, X_ini), m_(Y_ini, Y_ini)));
-    const double g2 = a_(m_(U_ini, U_ini), m_(V_ini, V_ini));
-    const double W = a_(g2, d_(m_(2.0, eps_th), r));
-    const double g_0 = __dsqrt_rn(W);
-    const double b_0 = d_(eps_th, W);
-    const double b = d_(fabs(Lz), g_0);
-    HypConsts c;
-    const double bg = m_(b_0, g_0);
-    c.theta_0 = d_atan2(fabs(Lz), bg);
-    const double den0 = __dsqrt_rn(a_(m_(m_(b_0, b_0), m_(g_0, g_0)), m_(Lz, Lz)));
-    c.cs_0 = d_(bg, den0);
-    c.sn_0 = d_(fabs(Lz), den0);
-    c.tn_0 = d_(fabs(Lz), bg);
-    d_sincos(0.5 * c.theta_0, &c.s0h, &c.c0h);
-    const double arg = a_(c.cs_0, d_(m_(b, c.sn_0), r));
-#else
     const double r_g = X_ini * U_ini + Y_ini * V_ini;
     const double Lz = X_ini * V_ini - Y_ini * U_ini;
-    const double r = sqrt(X_ini * X_ini + Y_ini * Y_ini);
+    const double aL = fabs(Lz);
+    const double r2 = X_ini * X_ini + Y_ini * Y_ini;
+    const double ir = rsqrt_normal(r2);
+    const double r = r2 * ir;
     const double g2 = U_ini * U_ini + V_ini * V_ini;
-    const double W = g2 + 2.0 * eps_th / r;
-    const double g_0 = sqrt(W);
-    const double b_0 = eps_th / W;
-    const double b = fabs(Lz) / g_0;
+    const double W = g2 + 2.0 * eps_th * ir;
+    const double ig_0 = rsqrt_normal(W);
+    const double g_0 = W * ig_0;
+    const double bg = eps_th * ig_0;           // b_0 g_0
+    const double b_g = bg * (ig_0 * ig_0);     // b_0 / g_0
+    const double g_b = g_0 * W * rcp_normal(eps_th);  // g_0 / b_0
+    const double b = aL * ig_0;
     HypConsts c;
-    const double bg = b_0 * g_0;
-    c.theta_0 = d_atan2(fabs(Lz), bg);
-    const double den0 = sqrt(b_0 * b_0 * (g_0 * g_0) + Lz * Lz);
-    c.cs_0 = bg / den0;
-    c.sn_0 = fabs(Lz) / den0;
-    c.tn_0 = fabs(Lz) / bg;
-    d_sincos(0.5 * c.theta_0, &c.s0h, &c.c0h);
-    const double arg = c.cs_0 + b * c.sn_0 / r;
-#endif
-    double theta_ini = (fabs(arg) > 1.0) ? 1e-30 : d_acos(arg);
-    if (Lz * r_g < 0.0) theta_ini = -theta_ini;
-    // state and dimensionless time at theta_ini (bia/find_hyperbola.f90:46-64)
+    const double iden0 = rsqrt_normal(bg * bg + Lz * Lz);
+    c.cs_0 = bg * iden0;
+    c.sn_0 = aL * iden0;
+    c.tn_0 = aL * (g_0 * rcp_normal(eps_th));
+    half_angle(c.sn_0, c.cs_0, c.s0h, c.c0h);
+    // the start: sine, cosine and angle
+    const double bs = b * c.sn_0;
+    const double D_i = bs * ir;  // cos theta - cos theta_0 = 2 sp sm
+    const double sgn = Lz > 0.0 ? 1.0 : -1.0;
+    double sn = sgn * (r_g * ir) * (c.sn_0 * ig_0), cs = c.cs_0 + D_i;
+    const double theta_ini = atan2(sn, cs);
+    const double inrm = rsqrt_normal(sn * sn + cs * cs);
+    sn *= inrm;
+    cs *= inrm;
     double sh, ch;
-    d_sincos(0.5 * theta_ini, &sh, &ch);
-    double sp_i, sm_i;
-    half_sines(c, theta_ini, sh, ch, sp_i, sm_i);
-    const double Dinv_i = 1.0 / (2.0 * sp_i * sm_i);
-#if BIA_REF_END_STATE
-    // the start position and the end state take sin and cos of the full angle, as the
-    // reference does: the end position is a difference of two positions of magnitude r,
-    // and only the same formula at both ends keeps their rounding from adding a bias
-    double sn, cs;
-    d_sincos(theta_ini, &sn, &cs);
-    const double x = r * cs, y = r * sn;
-    const double g0_sn0 = (Lz > 0.0) ? g_0 / c.sn_0 : -g_0 / c.sn_0;
-    const double u = g0_sn0 * (c.cs_0 * sn);
-    const double v = g0_sn0 * (1.0 - c.cs_0 * cs);
-    const double den_a = sqrt((X_ini * X_ini + Y_ini * Y_ini) * (x * x + y * y));
-    const double cs_a = (x * X_ini + y * Y_ini) / den_a;
-    const double sn_a = (x * Y_ini - y * X_ini) / den_a;
-#else
-    const double sn = 2.0 * sh * ch, cs = 1.0 - 2.0 * sh * sh;
-    const double x = r * cs, y = r * sn;
-    const double g0_sn0 = (Lz > 0.0) ? g_0 / c.sn_0 : -g_0 / c.sn_0;
-    const double u = g0_sn0 * (c.cs_0 * sn);
-    const double v = g0_sn0 * (1.0 - c.cs_0 * cs);
-    const double den_a = 1.0 / sqrt((X_ini * X_ini + Y_ini * Y_ini) * (x * x + y * y));
-    const double cs_a = (x * X_ini + y * Y_ini) * den_a;
-    const double sn_a = (x * Y_ini - y * X_ini) * den_a;
-#endif
-    const double tau_ini = c.tn_0 * sn * Dinv_i + d_log(sp_i / sm_i);
-    const double time_ini = tau_ini * b_0 / g_0;
-    const double time_end = (Lz > 0.0) ? time_ini + dt : time_ini - dt;
-    c.time_end_ = time_end * g_0 / b_0;
+    half_angle(sn, cs, sh, ch);
+    // sp sm = D_i / 2; the larger of the two is a sum without cancellation.  Away from the asymptotes the
+    // smaller one is taken from the angle too, as the iteration takes it: there rounding alone counts, and
+    // what start and end share cancels
+    const double big = c.s0h * ch + c.c0h * fabs(sh);
+    const double prod = D_i > 0.1 ? big * (c.s0h * ch - c.c0h * fabs(sh)) : 0.5 * D_i;
+    const double q_i = prod * rcp_normal(big * big);  // the smaller over the larger: sm/sp, or sp/sm for theta < 0
+    const double Dinv_i = 0.5 * rcp_normal(prod);
+    // state and dimensionless time there (bia/find_hyperbola.f90:46-64)
+    const double g0_cs0_sn0 = sgn * g_0 * c.cs_0 * rcp_normal(c.sn_0);
+    const double cs_a = (cs * X_ini + sn * Y_ini) * ir;
+    const double sn_a = (cs * Y_ini - sn * X_ini) * ir;
+    const double lq = log(q_i);
+    const double tau_ini = c.tn_0 * sn * Dinv_i + (sn >= 0.0 ? -lq : lq);
+    const double time_ini = tau_ini * b_g;
+    const double time_end = time_ini + sgn * dt;
+    c.time_end_ = time_end * g_b;
 
-    // two candidate starts (bia/find_hyperbola.f90:71-89): one Newton step from theta_ini
-    // (its residual is known already) and one from the atan guess
+    // the start of the iteration: one Newton step on (its residual is known already), or the guess
     const double error_ini_ = tau_ini - c.time_end_;
     const double d_ini = c.tn_0 * (1.0 - c.cs_0 * cs) * (Dinv_i * Dinv_i) + c.sn_0 * Dinv_i;
-    const double th_ini_end = (error_ini_ == 0.0) ? theta_ini : theta_ini - error_ini_ / d_ini;
-    const double theta_gss = 2.0 / kPi * c.theta_0 * d_atan(c.time_end_ / c.tn_0);
-    double error_gss_, d_gss, spg, smg;
-    hyp_eval(c, theta_gss, error_gss_, d_gss, spg, smg);
-    const double th_gss_end = (error_gss_ == 0.0) ? theta_gss : theta_gss - error_gss_ / d_gss;
-    double theta_end, error_;
-    if (fabs(error_gss_) > 10.0 * fabs(error_ini_)) {
-        theta_end = th_ini_end;
-        error_ = error_ini_;
+    const double step_ini = error_ini_ * rcp_normal(d_ini);
+    double theta_end = (error_ini_ == 0.0) ? theta_ini : theta_ini - step_ini;
+    double error_ = error_ini_;
+    if (fabs(step_ini) <= 1e-3 * (big * q_i)) {  // big q_i: the sine of half the smaller distance
+        // on from the Newton step by theta(t)'s Taylor series to third order (theta' = L/r^2,
+        // r'' = L^2/r^3 + eps/r^2): the first evaluation then meets the rounding floor
+        const double rho = r_g * (ir * ir) * dt;
+        const double kap = (Lz * Lz * ir + eps_th) * (ir * ir * ir) * (dt * dt);
+        theta_end = theta_ini - step_ini * (1.0 + (rho * rho - rho - kap * (1.0 / 3.0)));
     } else {
-        theta_end = th_gss_end;
-        error_ = error_gss_;
+        double error_gss_;
+        const double th_gss_end = hyp_guess(c, &error_gss_);
+        if (!(fabs(error_gss_) > 10.0 * fabs(error_ini_))) {
+            theta_end = th_gss_end;
+            error_ = error_gss_;
+        }
     }
     // minimum-residual Newton loop with cycle detection (bia/find_hyperbola.f90:93-120).
     // The reference compares each residual with every earlier one (error_restore_); here
@@ -338,6 +337,8 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
     double best_res = fabs(error_);
     const double kNoResidual = __longlong_as_double(0x7ff8000000000000LL);  // compares unequal
     double h0 = kNoResidual, h1 = kNoResidual, h2 = kNoResidual, h3 = kNoResidual;
+    // A Newton step of at most four ulps of the angle ends it too: what follows would be the residuals'
+    // rounding, on a few of the warp's lanes.
     int IR = 0;
     *bracket_exit = 0;
     while (IR < ITR) {
@@ -349,7 +350,7 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
             break;
         }
         error_ = e;
-        theta_end = (e == 0.0) ? theta_now : theta_now - e / d;
+        theta_end = (e == 0.0) ? theta_now : theta_now - e * rcp_normal(d);
         IR++;
         if (error_ == h0 || error_ == h1 || error_ == h2 || error_ == h3) break;
         h3 = h2;
@@ -358,33 +359,26 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
         h0 = error_;
         best_res = fmin(best_res, fabs(error_));
         if (fabs(error_) < fabs(err_stock)) {
-            err_stock = error_ * b_0 / g_0;
+            err_stock = error_ * b_g;
             theta_stock = theta_end;
             if (fabs(err_stock) < 2e-16) break;
         }
+        if (fabs(theta_end - theta_now) <= kFewUlps * fabs(theta_now)) break;
     }
-    *error_end = error_ * b_0 / g_0;
+    *error_end = error_ * b_g;
     *fallback = 0;
     if (!(best_res <= 1e-8 * (1.0 + fabs(c.time_end_)))) {  // the reference loop did not converge
         theta_stock = hyp_safe(c, theta_stock);
         *fallback = 1;
     }
-    // end state (bia/find_hyperbola.f90:126-142)
-#if BIA_REF_END_STATE
+    // end state (bia/find_hyperbola.f90:126-142): sine and cosine of the full angle, as the reference
+    // takes them
     double sn_end, cs_end;
-    d_sincos(theta_stock, &sn_end, &cs_end);
-    const double r_end = b * c.sn_0 / (cs_end - c.cs_0);
-#else
-    d_sincos(0.5 * theta_stock, &sh, &ch);
-    const double sn_end = 2.0 * sh * ch, cs_end = 1.0 - 2.0 * sh * sh;
-    double sp_e, sm_e;
-    half_sines(c, theta_stock, sh, ch, sp_e, sm_e);
-    const double r_end = b * c.sn_0 / (2.0 * sp_e * sm_e);
-#endif
-    const double u_end = g0_sn0 * c.cs_0 * sn_end;
-    const double du_end = u_end - u;
-    const double v_end = g0_sn0 * (1.0 - c.cs_0 * cs_end);
-    const double dv_end = v_end - v;
+    sincos(theta_stock, &sn_end, &cs_end);
+    const double r_end = bs * rcp_normal(cs_end - c.cs_0);
+    // velocity (g_0/sin theta_0) (cos theta_0 sin theta, 1 - cos theta_0 cos theta): its change
+    const double du_end = g0_cs0_sn0 * (sn_end - sn);
+    const double dv_end = g0_cs0_sn0 * (cs - cs_end);
     YN[0] = r_end * (cs_end * cs_a - sn_end * sn_a);
     YN[1] = r_end * (cs_end * sn_a + sn_end * cs_a);
     YN[2] = YZ[2] + (du_end * cs_a - dv_end * sn_a);
@@ -406,7 +400,7 @@ static __device__ __noinline__ double kepler_safe(double M, double e, double x)
     if (!(x >= lo && x <= hi)) x = M;
     for (int it = 0; it < 400; it++) {
         double sx, cx;
-        d_sincos(x, &sx, &cx);
+        sincos(x, &sx, &cx);
         const double f = x - e * sx - M;
         if (f == 0.0) break;
         if (f < 0.0) lo = x; else hi = x;
@@ -418,48 +412,55 @@ static __device__ __noinline__ double kepler_safe(double M, double e, double x)
     return x;
 }
 
-#ifndef BIA_INLINE_ELLIPSE
-#define BIA_INLINE_ELLIPSE 0
-#endif
-#if BIA_INLINE_ELLIPSE
-#define BIA_ELLIPSE_LINKAGE __device__ __forceinline__
-#else
-#define BIA_ELLIPSE_LINKAGE static __device__ __noinline__
-#endif
-BIA_ELLIPSE_LINKAGE int ellipse(double eps_th, double dt, int ITR, const double YZ[4], double YN[4],
+static __device__ __noinline__ int ellipse(double eps_th, double dt, int ITR, const double YZ[4], double YN[4],
                                 double *error, int *fallback)
 {
     const double X_ini = YZ[0], Y_ini = YZ[1], U_ini = YZ[2], V_ini = YZ[3];
     const double g2_ini = U_ini * U_ini + V_ini * V_ini;
-    const double r_ini = sqrt(X_ini * X_ini + Y_ini * Y_ini);
-    const double W = g2_ini + 2.0 * eps_th / r_ini;
+    const double r2 = X_ini * X_ini + Y_ini * Y_ini;
+    const double ir = rsqrt_normal(r2);
+    const double r_ini = r2 * ir;
+    const double W = g2_ini + 2.0 * eps_th * ir;
     const double L = X_ini * V_ini - Y_ini * U_ini;
     const double r_g_ini = X_ini * U_ini + Y_ini * V_ini;
-    const double g_a = f_sign(sqrt(-W), L);
-    const double a = eps_th / W;
-    const double b = L / g_a;
-    const double omega_a = g_a / a;
-    double ecc = sqrt((a * g_a) * (a * g_a) - L * L) / (a * g_a);
-    double xi_ini;
+    const double iga = f_sign(rsqrt_normal(-W), L);  // 1 / g_a
+    const double g_a = -W * iga;
+    const double a = -eps_th * (iga * iga);
+    const double b = L * iga;
+    const double ia = W * rcp_normal(eps_th);
+    const double omega_a = g_a * ia;
+    // the start's eccentric anomaly E, its sine and cosine and the eccentricity from the state itself:
+    // a e (sin E, cos E) = (r.g / g_a, a - r).  (The reference's sqrt((a g_a)^2 - L^2) / (a g_a) is off by
+    // 1e-8 on a circular orbit, and not of one piece with the angle.)
+    double ecc = fabs(a - r_ini) * ia;
+    double xi_ini, s_ini, c_ini;
+    bool from_angle = false;
     if (r_g_ini == 0.0) {
         if (r_ini < a) {
             xi_ini = 0.0;
         } else if (r_ini == a) {
-            xi_ini = d_atan2(Y_ini, X_ini);
+            xi_ini = atan2(Y_ini, X_ini);
             ecc = 0.0;
         } else {
             xi_ini = f_sign(kPi, L);
         }
+        from_angle = true;
     } else {
-        xi_ini = d_atan2(r_g_ini / g_a, a - r_ini);
+        s_ini = r_g_ini * iga;
+        c_ini = a - r_ini;
+        xi_ini = atan2(s_ini, c_ini);
+        const double n2 = s_ini * s_ini + c_ini * c_ini;
+        const double in = rsqrt_normal(n2);
+        s_ini *= in;
+        c_ini *= in;
+        ecc = n2 * in * ia;
+        from_angle = !(n2 > 1e-290);
+        if (from_angle) ecc = sqrt(n2) * ia;
     }
-    double s_ini, c_ini;
-    d_sincos(xi_ini, &s_ini, &c_ini);
-    const double alpha = d_atan2(Y_ini, X_ini) - d_atan2(b * s_ini, a * (c_ini - ecc));
+    if (from_angle) sincos(xi_ini, &s_ini, &c_ini);
+    const double px = a * (c_ini - ecc), py = b * s_ini;  // the start in the orbit's frame
     const double tau_ini = xi_ini - ecc * s_ini;
-    const double time_ini = tau_ini / omega_a;
-    const double time_end = time_ini + dt;
-    const double tau_end = omega_a * time_end;
+    const double tau_end = fma(omega_a, dt, tau_ini);
     *error = 0.0;
     if (dt == 0.0) {
 #pragma unroll
@@ -470,35 +471,48 @@ BIA_ELLIPSE_LINKAGE int ellipse(double eps_th, double dt, int ITR, const double 
     // (bia/find_ellipse.f90:106-157).  Start: one Newton step from the initial anomaly
     // xi_ini, whose residual is omega dt, instead of the reference's start from the mean
     // anomaly (xi_2 + delta_ini, bia/find_ellipse.f90:116-129), which needs ~8 steps on
-    // average and fails outright for e near 1; the root is the same.
-    int ir = 0;
+    // average and fails outright for e near 1; the root is the same.  A small step goes on by the
+    // reversion of q x + (e s/2) x^2 + (e c/6) x^3 - ... = omega dt, q = 1 - e c, to fourth order, and the
+    // first evaluation meets the rounding floor.  A Newton step of at most four ulps ends the loop, and
+    // the end state turns the last iterate's sine and cosine by the last step.
+    int ir_ = 0;
     const double error_ini = tau_end - xi_ini + ecc * s_ini;
     double xi_2 = xi_ini;
     double error_tm2 = error_ini;
-    double s2, c2, delta_xi2;
-    double xi = xi_ini + error_ini / (1.0 - ecc * c_ini);
+    double s2 = s_ini, c2 = c_ini;
+    const double iq = rcp_normal(1.0 - ecc * c_ini);
+    double xi = error_ini * iq;
+    if (fabs(xi) <= 1e-2) {
+        const double A = 0.5 * ecc * s_ini * iq, B = (1.0 / 6.0) * ecc * c_ini * iq;
+        const double A2 = A * A;
+        xi *= 1.0 + xi * (xi * (2.0 * A2 - B + xi * A * (5.0 * (B - A2) + 1.0 / 12.0)) - A);
+    }
+    xi = xi_ini + xi;
     double xi_1 = __longlong_as_double(0x7ff8000000000000LL);  // unset: compares unequal
     double error_tm1 = error_tm2;
+    double last = 1.0;  // the step from the iterate whose sine and cosine are s2, c2
     bool conv = false;
-    while (xi_1 != xi_2 && ir <= ITR) {
-        ir++;
+    while (xi_1 != xi_2 && ir_ <= ITR) {
+        ir_++;
         xi_1 = xi;
-        double s1, c1;
-        d_sincos(xi_1, &s1, &c1);
-        error_tm1 = tau_end - xi_1 + ecc * s1;
-        xi = xi_1 + error_tm1 / (1.0 - ecc * c1);
-        if (error_tm1 == 0.0 || error_tm1 == error_tm2 || error_tm1 + error_tm2 == 0.0) {
+        sincos(xi_1, &s2, &c2);
+        error_tm1 = tau_end - xi_1 + ecc * s2;
+        last = error_tm1 * rcp_normal(1.0 - ecc * c2);
+        xi = xi_1 + last;
+        if (error_tm1 == 0.0 || error_tm1 == error_tm2 || error_tm1 + error_tm2 == 0.0 ||
+            fabs(last) <= kFewUlps * fabs(xi_1)) {
             *error = error_tm1;
             conv = true;
             break;
         }
-        ir++;
+        ir_++;
         xi_2 = xi;
-        d_sincos(xi_2, &s2, &c2);
+        sincos(xi_2, &s2, &c2);
         error_tm2 = tau_end - xi_2 + ecc * s2;
-        delta_xi2 = error_tm2 / (1.0 - ecc * c2);
-        xi = xi_2 + delta_xi2;
-        if (error_tm2 == 0.0 || error_tm1 == error_tm2 || error_tm1 + error_tm2 == 0.0) {
+        last = error_tm2 * rcp_normal(1.0 - ecc * c2);
+        xi = xi_2 + last;
+        if (error_tm2 == 0.0 || error_tm1 == error_tm2 || error_tm1 + error_tm2 == 0.0 ||
+            fabs(last) <= kFewUlps * fabs(xi_2)) {
             *error = error_tm2;
             conv = true;
             break;
@@ -509,21 +523,30 @@ BIA_ELLIPSE_LINKAGE int ellipse(double eps_th, double dt, int ITR, const double 
     if (!conv && !(fmin(fabs(error_tm1), fabs(error_tm2)) <= 1e-8 * (1.0 + fabs(tau_end)))) {
         xi = kepler_safe(tau_end, ecc, xi);
         *fallback = 1;
+        last = 1.0;
     }
     double sn_end, cs_end;
-    d_sincos(xi, &sn_end, &cs_end);
+    if (fabs(last) <= 1e-8) {  // xi = last iterate + last, to the second order (the next is 1e-24)
+        const double h2 = 1.0 - 0.5 * last * last;
+        sn_end = fma(s2, h2, c2 * last);
+        cs_end = fma(c2, h2, -s2 * last);
+    } else {
+        sincos(xi, &sn_end, &cs_end);
+    }
     const double xx_end = a * (cs_end - ecc);
     const double yy_end = b * sn_end;
-    const double rr_end = a * (1.0 - ecc * cs_end);
-    const double uu_end = -a * g_a * sn_end / rr_end;
-    const double vv_end = b * g_a * cs_end / rr_end;
-    double sn_alp, cs_alp;
-    d_sincos(alpha, &sn_alp, &cs_alp);
+    const double gr = g_a * rcp_normal(1.0 - ecc * cs_end);  // a g_a / r
+    const double uu_end = -gr * sn_end;
+    const double vv_end = b * ia * gr * cs_end;
+    // the rotation from the orbit's frame: the start's position in both (the reference takes the
+    // difference of the two angles by atan2, and its sine and cosine back)
+    const double in = rsqrt_normal((px * px + py * py) * r2);
+    const double cs_alp = (px * X_ini + py * Y_ini) * in, sn_alp = (px * Y_ini - py * X_ini) * in;
     YN[0] = xx_end * cs_alp - yy_end * sn_alp;
     YN[1] = xx_end * sn_alp + yy_end * cs_alp;
     YN[2] = uu_end * cs_alp - vv_end * sn_alp;
     YN[3] = uu_end * sn_alp + vv_end * cs_alp;
-    return ir;
+    return ir_;
 }
 
 // ---------------------------------------------------------------------------
@@ -616,30 +639,6 @@ struct Fehlberg {
     static constexpr double DA1 = 1.0 / 360, DA3 = -128.0 / 4275, DA4 = -2197.0 / 75240,
                             DA5 = 1.0 / 50, DA6 = 2.0 / 55;
 };
-
-// 1/sqrt(x) of a normal x: the hardware approximation and one step
-// of Householder's third-order iteration y (1 + e/2 + 3/8 e^2), e = 1 - x y^2 (measured
-// at most 2^-19.04 over 1e9 values; the next term, 5/16 e^3, is below 3e-18).  Zero, subnormal
-// and infinite x give NaN or infinity: its callers test for them.
-__device__ __forceinline__ double rsqrt_normal(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-__dmul_rn(x, y), y, 1.0);
-    return fma(fma(e, 0.375, 0.5), __dmul_rn(y, e), y);
-}
-
-// c x^(-3/2) of a normal x from the same approximation y, whose square is exact (its low half is zero):
-// c y^3 (1 + 3/2 e + 15/8 e^2), e = 1 - x y^2; the next term, 35/16 e^3, is below 3e-17.
-__device__ __forceinline__ double scaled_rsqrt3_normal(double c, double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double y2 = y * y;
-    const double e = fma(-x, y2, 1.0);
-    const double c3 = (c * y) * y2;
-    return fma(c3 * e, fma(e, 1.875, 1.5), c3);
-}
 
 // Acceleration (ax, ay) = eps (x, y) / r^3 of moon_2D.  kNormal: eps r^-3 from one reciprocal square
 // root (x^2 + y^2 a normal number), at about half the FP64 instructions of the reference's
@@ -1268,8 +1267,10 @@ __device__ __forceinline__ int alg_classify(double eps_ij, const double r[3], co
     const double L1 = r[2] * g[0] - r[0] * g[2];
     const double L2 = r[0] * g[1] - r[1] * g[0];
     const double Lsq = L0 * L0 + L1 * L1 + L2 * L2;
-    const double r_ij = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-    const double E_ij = gsq + 2.0 * eps_ij / r_ij;
+    const double rsq = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+    double E_ij = gsq + 2.0 * eps_ij * rsqrt_normal(rsq);
+    // near zero (a parabola is E == 0 exactly) and beyond the approximation's range, the root and division
+    if (!(fabs(E_ij) > 1e-12 * gsq && rsq > 1e-290)) E_ij = gsq + 2.0 * eps_ij / sqrt(rsq);
     E_out = E_ij;
     Lsq_out = Lsq;
     if (E_ij == 0.0) return kClsPar;
