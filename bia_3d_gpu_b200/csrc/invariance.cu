@@ -6,12 +6,13 @@
 // (q_i q_j / r_ij).  The reference's inv_device gives thread i the whole row j > i
 // (triangular imbalance, uncoalesced) and sum_device runs 11 serial sums on one thread
 // each.  Here the pair sum uses the step kernel's 32 x 32 warp-blocks over the upper
-// triangle with shuffled column data, each warp's partial goes to a fixed slot, and all
-// partials are reduced by a tree in fixed order, so the result is reproducible and the
-// rounding error grows with log(n) instead of n.
+// triangle, each CTA's partial goes to a fixed slot, and all partials are added in a
+// fixed order, so the result is reproducible; a lane sums 32 pairs of a block, then blocks, then
+// lanes, warps and CTAs, so that the rounding error stays far below n ulps.
 #include <cuda_runtime.h>
 
 #include "bia_internal.cuh"
+#include "bia_pair.cuh"
 
 namespace bia {
 
@@ -25,139 +26,167 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// per-block partials of the ten one-body sums, order {KE, -, Lx, Ly, Lz, Ua, Va, Wa, Xa, Ya, Za}
-__global__ void __launch_bounds__(kInvThreads) inv_onebody_kernel(int n, const double *x, const double *y,
-                                                                  const double *z, const double *u,
-                                                                  const double *v, const double *w,
-                                                                  double *part /* [blocks][11] */)
+// Unit t of the pair sum: block rows 2 g and 2 g + 1 (as far as they are <= bj) of block column bj; the
+// columns before bj hold floor((bj + 1)^2 / 4) units.
+__host__ __device__ __forceinline__ long long inv_units_before(long long bj) { return (bj + 1) * (bj + 1) / 4; }
+
+__device__ __forceinline__ void inv_unit_coords(long long t, int &g, int &bj)
 {
-    __shared__ double sh[kInvWarps][11];
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    double s[11];
-#pragma unroll
-    for (int k = 0; k < 11; k++) s[k] = 0.0;
-    if (p < n) {
-        const double X = x[p], Y = y[p], Z = z[p], U = u[p], V = v[p], W = w[p];
-        s[0] = U * U + V * V + W * W;
-        s[2] = Y * W - Z * V;
-        s[3] = Z * U - X * W;
-        s[4] = X * V - Y * U;
-        s[5] = U; s[6] = V; s[7] = W;
-        s[8] = X; s[9] = Y; s[10] = Z;
+    long long c = (long long)(2.0 * sqrt((double)t));
+    while (inv_units_before(c) > t) c--;
+    while (inv_units_before(c + 1) <= t) c++;
+    bj = (int)c;
+    g = (int)(t - inv_units_before(c));
+}
+
+// The lane's pairs of a block with roots and divisions: coincident, subnormal or overflowing separations.
+static __device__ __noinline__ double inv_block_again(const double2 *xy, const double2 *zq, double xi, double yi, double zi,
+                                                      double qi, int lane, bool diag, bool row_live, int ncols)
+{
+    double acc = 0.0;
+    for (int k = diag ? 1 : 0; k <= (diag ? 16 : 31); k++) {
+        const int src = (lane + k) & 31;
+        if ((!diag || k < 16 || lane < 16) && row_live && src < ncols) {
+            const double dx = xi - xy[src].x, dy = yi - xy[src].y, dz = zi - zq[src].x;
+            acc += qi * zq[src].y * (1.0 / sqrt(dx * dx + dy * dy + dz * dz));
+        }
     }
+    return acc;
+}
+
+// The invariants in one launch: every CTA takes its share of the particles (the ten one-body sums) and of the
+// pair sum (q_i q_j) / r_ij over i<j (one warp a unit of two 32 x 32 blocks of one block column), leaves its
+// twelve sums in part[blockIdx.x][12], and the CTA that arrives last adds them up, one warp a sum, in block
+// order: the result does not depend on which CTA that is.  out[12], order {KE, -, Lx, Ly, Lz, Ua, Va, Wa,
+// Xa, Ya, Za, pair sum}.
+//
+// A pair is a distance and a reciprocal square root, 12 FP64 operations (28 register-read cycles a warp).
+// Its column comes from two 16-byte shared-memory rows, eight cycles of the SM's one shared-memory port per
+// scheduler, so a lane keeps two rows and reads a column once for both.  n = 32768: 1.46 ms with shuffled
+// columns, 1/sqrt and one partial per 8 blocks added by a single CTA, 0.70 with one row a lane, 0.57 so.
+__global__ void __launch_bounds__(kInvThreads) inv_kernel(int n, long long units, const double *x, const double *y,
+                                                          const double *z, const double *u, const double *v,
+                                                          const double *w, const double *q, double *part,
+                                                          unsigned int *arrived, double *out)
+{
+    __shared__ double sh[kInvWarps][12];
+    __shared__ double2 s_xy[kInvWarps][32], s_zq[kInvWarps][32];
+    __shared__ bool s_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double2 *xy = s_xy[wid], *zq = s_zq[wid];
+    double pairs = 0.0;
+    for (long long t = (long long)blockIdx.x * kInvWarps + wid; t < units; t += (long long)gridDim.x * kInvWarps) {
+        int g, bj;
+        inv_unit_coords(t, g, bj);
+        const int jo = bj * 32 + lane, ncols = n - bj * 32;
+        const bool jv = jo < n;
+        double xi[2], yi[2], zi[2], qi[2];
+        bool iv[2];
 #pragma unroll
-    for (int k = 0; k < 11; k++) {
-        double t = warp_sum(s[k]);
+        for (int h = 0; h < 2; h++) {
+            const int i = (2 * g + h) * 32 + lane;
+            iv[h] = 2 * g + h <= bj && i < n;
+            xi[h] = iv[h] ? x[i] : 0.0;
+            yi[h] = iv[h] ? y[i] : 0.0;
+            zi[h] = iv[h] ? z[i] : 0.0;
+            qi[h] = iv[h] ? (q ? q[i] : 1.0) : 0.0;
+        }
+        __syncwarp();
+        xy[lane] = make_double2(jv ? x[jo] : 0.0, jv ? y[jo] : 0.0);
+        zq[lane] = make_double2(jv ? z[jo] : 0.0, jv ? (q ? q[jo] : 1.0) : 0.0);
+        __syncwarp();
+        double a[2] = {0.0, 0.0};
+        if (2 * g + 1 < bj && ncols >= 32) {  // two blocks off the diagonal, every pair there
+#pragma unroll 4
+            for (int k = 0; k < 32; k++) {
+                const int src = (lane + k) & 31;
+                const double2 cxy = xy[src], czq = zq[src];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const double dx = xi[h] - cxy.x, dy = yi[h] - cxy.y, dz = zi[h] - czq.x;
+                    a[h] = fma(czq.y, rsqrt_normal(fma(dz, dz, fma(dy, dy, dx * dx))), a[h]);
+                }
+            }
+        } else {
+            for (int h = 0; h < 2; h++) {
+                const bool diag = 2 * g + h == bj;
+                for (int k = diag ? 1 : 0; k <= (diag ? 16 : 31); k++) {
+                    const int src = (lane + k) & 31;
+                    const double2 cxy = xy[src], czq = zq[src];
+                    const double dx = xi[h] - cxy.x, dy = yi[h] - cxy.y, dz = zi[h] - czq.x;
+                    const double r = rsqrt_normal(fma(dz, dz, fma(dy, dy, dx * dx)));
+                    if ((!diag || k < 16 || lane < 16) && iv[h] && src < ncols) a[h] = fma(czq.y, r, a[h]);
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            double acc = qi[h] * a[h];
+            if (!isfinite(acc))
+                acc = inv_block_again(xy, zq, xi[h], yi[h], zi[h], qi[h], lane, 2 * g + h == bj, iv[h], ncols);
+            pairs += acc;
+        }
+    }
+    double s[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) s[k] = 0.0;
+    s[11] = pairs;
+    for (int p = blockIdx.x * kInvThreads + threadIdx.x; p < n; p += gridDim.x * kInvThreads) {
+        const double X = x[p], Y = y[p], Z = z[p], U = u[p], V = v[p], W = w[p];
+        s[0] += U * U + V * V + W * W;
+        s[2] += Y * W - Z * V;
+        s[3] += Z * U - X * W;
+        s[4] += X * V - Y * U;
+        s[5] += U; s[6] += V; s[7] += W;
+        s[8] += X; s[9] += Y; s[10] += Z;
+    }
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+        const double t = warp_sum(s[k]);
         if (lane == 0) sh[wid][k] = t;
     }
     __syncthreads();
-    if (threadIdx.x < 11) {
+    if (threadIdx.x < 12) {
         double t = 0.0;
         for (int k = 0; k < kInvWarps; k++) t += sh[k][threadIdx.x];
-        part[(size_t)blockIdx.x * 11 + threadIdx.x] = t;
+        part[(size_t)blockIdx.x * 12 + threadIdx.x] = t;
+        __threadfence();
     }
-}
-
-__device__ __forceinline__ void inv_block_coords(long long t, int &bi, int &bj)
-{
-    long long c = (long long)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while (c * (c + 1) / 2 > t) c--;
-    while ((c + 1) * (c + 2) / 2 <= t) c++;
-    bj = (int)c;
-    bi = (int)(t - c * (c + 1) / 2);
-}
-
-// sum over i<j of (q_i q_j) / r_ij; one warp per 32 x 32 block, one partial per CTA
-__global__ void __launch_bounds__(kInvThreads) inv_pairs_kernel(int n, long long nwb, const double *x,
-                                                                const double *y, const double *z,
-                                                                const double *q, double *part)
-{
-    __shared__ double sh[kInvWarps];
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const long long t = (long long)blockIdx.x * kInvWarps + wid;
-    double acc = 0.0;
-    if (t < nwb) {
-        int bi, bj;
-        inv_block_coords(t, bi, bj);
-        const int i = bi * 32 + lane, jo = bj * 32 + lane;
-        const bool iv = i < n, jv = jo < n;
-        const double xi = iv ? x[i] : 0.0, yi = iv ? y[i] : 0.0, zi = iv ? z[i] : 0.0;
-        const double qi = (iv && q) ? q[i] : 1.0;
-        const double xj = jv ? x[jo] : 0.0, yj = jv ? y[jo] : 0.0, zj = jv ? z[jo] : 0.0;
-        const double qj = (jv && q) ? q[jo] : 1.0;
-        const bool diag = bi == bj;
-        const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
-        for (int k = k0; k <= k1; k++) {
-            const int src = (lane + k) & 31;
-            const double cx = __shfl_sync(full, xj, src);
-            const double cy = __shfl_sync(full, yj, src);
-            const double cz = __shfl_sync(full, zj, src);
-            const double cq = __shfl_sync(full, qj, src);
-            const int j = bj * 32 + src;
-            if ((!diag || k < 16 || lane < 16) && iv && j < n) {
-                const double dx = xi - cx, dy = yi - cy, dz = zi - cz;
-                const double w = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
-                acc += q ? qi * cq * w : w;
-            }
-        }
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) sh[wid] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < kInvWarps; k++) s += sh[k];
-        part[blockIdx.x] = s;
+    if (threadIdx.x == 0) s_last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int k = wid; k < 12; k += kInvWarps) {
+        double t = 0.0;
+        for (unsigned int b = lane; b < gridDim.x; b += 32) t += __ldcg(part + (size_t)b * 12 + k);
+        t = warp_sum(t);
+        if (lane == 0) out[k] = t;
     }
 }
 
-// fixed-order tree reduction of `count` groups of `width` values: out[k] = sum_g in[g*width+k]
-__global__ void __launch_bounds__(1024) inv_final_kernel(const double *in, long long count, int width,
-                                                         double *out)
+// Grid: enough CTAs for the pair units, at most what is resident (4 per SM).
+static int inv_grid(int n)
 {
-    __shared__ double sh[32];
-    for (int k = 0; k < width; k++) {
-        double s = 0.0;
-        for (long long g = threadIdx.x; g < count; g += blockDim.x) s += in[g * width + k];
-        s = warp_sum(s);
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            double t = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : 0.0;
-            t = warp_sum(t);
-            if (threadIdx.x == 0) out[k] = t;
-        }
-        __syncthreads();
-    }
+    const long long blocks = (inv_units_before((n + 31) / 32) + kInvWarps - 1) / kInvWarps;
+    const int sms = device_sm_count();
+    const long long cap = sms > 0 ? 4LL * sms : 592;
+    return (int)(blocks < cap ? blocks : cap);
 }
 
-// Enqueue the invariants of device SoA state into out_dev[12] (11 values, slot 1 = raw
+// Enqueue the invariants of device SoA state into out_dev[12] (11 values, slot 1 = 0, slot 11 = raw
 // pair sum before the eps_th factor).  scratch must hold inv_scratch_doubles(n).
-size_t inv_scratch_doubles(int n)
-{
-    const long long nb = (n + 31) / 32;
-    const long long nwb = nb * (nb + 1) / 2;
-    const long long pair_blocks = (nwb + kInvWarps - 1) / kInvWarps;
-    const long long one_blocks = (n + kInvThreads - 1) / kInvThreads;
-    return (size_t)(one_blocks * 11 + pair_blocks + 16);
-}
+size_t inv_scratch_doubles(int n) { return (size_t)inv_grid(n) * 12 + 1; }
 
 cudaError_t enqueue_invariance(cudaStream_t st, int n, const double *x, const double *y, const double *z,
                                const double *u, const double *v, const double *w, const double *q,
                                double *scratch, double *out_dev)
 {
-    const long long nb = (n + 31) / 32;
-    const long long nwb = nb * (nb + 1) / 2;
-    const long long pair_blocks = (nwb + kInvWarps - 1) / kInvWarps;
-    const int one_blocks = (n + kInvThreads - 1) / kInvThreads;
-    double *p1 = scratch;
-    double *p2 = scratch + (size_t)one_blocks * 11;
-    inv_onebody_kernel<<<one_blocks, kInvThreads, 0, st>>>(n, x, y, z, u, v, w, p1);
-    inv_pairs_kernel<<<(unsigned)pair_blocks, kInvThreads, 0, st>>>(n, nwb, x, y, z, q, p2);
-    inv_final_kernel<<<1, 1024, 0, st>>>(p1, one_blocks, 11, out_dev);
-    inv_final_kernel<<<1, 1024, 0, st>>>(p2, pair_blocks, 1, out_dev + 11);
+    const int grid = inv_grid(n);
+    unsigned int *arrived = (unsigned int *)(scratch + (size_t)grid * 12);
+    cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), st);
+    if (e != cudaSuccess) return e;
+    inv_kernel<<<grid, kInvThreads, 0, st>>>(n, inv_units_before((n + 31) / 32), x, y, z, u, v, w, q, scratch, arrived, out_dev);
     return cudaGetLastError();
 }
 
