@@ -59,6 +59,7 @@ __device__ __forceinline__ bool learned_candidate(double eps_ij, double dt, cons
 // division, no root).  Ellipses with e^2 < 0.9 and attractive hyperbolae with
 // 1.1 < e^2 <= 2500 (the universal-variable band of alg_classify, |e^2 - 1| < 0.1, and the
 // hyperbolic head's e <= 50); radial (L = 0), zero-velocity and parabolic pairs have e = 1.
+// learned_prepare decides the rest (e as the heads take it, |M1| <= 100).
 // Returns kLearnedEll, kLearnedHyp or kLearnedPlain; e2m = e^2 mu^2.
 __device__ __forceinline__ int learned_band(const UvPair &p, double dt, double &e2m)
 {
@@ -92,9 +93,9 @@ __device__ __forceinline__ void learned_prepare(double eps_ij, double dt, const 
     }
     // one rsqrt and one reciprocal for the elements (|beta| > 0 inside the bands)
     const double ab = fabs(L.p.beta);
-    L.isqb = rsqrt(ab);
+    L.isqb = rsqrt_normal(ab);
     L.sqb = ab * L.isqb;
-    const double imu = 1.0 / L.p.mu;
+    const double imu = rcp_normal(L.p.mu);
     const double c0m = L.p.r0 * ab * imu;
     const double s0 = L.p.sig * L.sqb * imu;
     const double n_dt = ab * L.sqb * imu * dt;
@@ -133,23 +134,6 @@ __device__ __forceinline__ void learned_prepare(double eps_ij, double dt, const 
         L.unfold_shift = 0.0f;
         L.kind = kLearnedHyp;
     }
-}
-
-// The heads' domain as a cheap test on the universal-variable quantities of the pair (the
-// split step's filter that sends a pair to the learned kernel): learned_band, then for the
-// hyperbolae in the band |M1| <= 100 in FP32.  The learned kernel decides again with
-// learned_prepare (the same band, |M1| from its own elements) and solves a pair outside
-// its domain with the plain solver, so this test only chooses the kernel.
-__device__ __forceinline__ bool learned_filter(const UvPair &p, double dt)
-{
-    double e2m;
-    const int band = learned_band(p, dt, e2m);
-    if (band != kLearnedHyp) return band == kLearnedEll;
-    const float mu = (float)p.mu, ab = (float)(-p.beta), sqb = sqrtf(ab);
-    const float s0 = (float)p.sig * sqb / mu;
-    const float e = sqrtf((float)e2m) / mu;
-    const float M1 = s0 - asinhf(s0 / e) + ab * sqb / mu * (float)dt;
-    return fabsf(M1) <= kHypMMax;
 }
 
 // x - sin x and sinh x - x without cancellation (FP32): series below 0.5

@@ -69,7 +69,7 @@ __device__ __forceinline__ void cta_scan2(MlpSmem &S, int a, int b, int &oa, int
 // The split learned step in three kernels, shared by the single-system step and the ensemble:
 //  rest    the walk of the universal-variable step (bia_uv_walk.cuh): short-step pairs on the spot;
 //          of the others, a pair whose fifth-order start is exact is composed, one whose start is
-//          not exact and that lies inside a head's domain (learned_filter, then learned_prepare)
+//          not exact and that lies inside a head's domain (learned_band, then learned_prepare)
 //          is deferred, the rest run the safeguarded Newton iteration.  Deferred pairs get rows in
 //          the global row buffer of each head and their warp-block a list entry: from a warp's queue, with
 //          one atomic per head for the whole queue; from a block finished on the spot
@@ -120,7 +120,8 @@ static __device__ __noinline__ int rest_pair(double eps_ij, double dt, double rx
     const UvPair p = uv_prepare(eps_ij, r, g);
     if (dt == 0.0) return kLearnedPlain;  // h stays zero
     const UvSeries sq = uv_series(p, dt);
-    if (!sq.exact && learned_filter(p, dt)) {
+    double e2m;
+    if (!sq.exact && learned_band(p, dt, e2m) != kLearnedPlain) {  // learned_prepare tests the rest of the domain
         LearnedPair L;
         learned_prepare(eps_ij, dt, r, g, L);
         if (L.kind != kLearnedPlain) {

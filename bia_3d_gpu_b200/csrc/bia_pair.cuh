@@ -262,7 +262,6 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
     const double aL = fabs(Lz);
     const double r2 = X_ini * X_ini + Y_ini * Y_ini;
     const double ir = rsqrt_normal(r2);
-    const double r = r2 * ir;
     const double g2 = U_ini * U_ini + V_ini * V_ini;
     const double W = g2 + 2.0 * eps_th * ir;
     const double ig_0 = rsqrt_normal(W);
@@ -957,8 +956,7 @@ __device__ __forceinline__ double uv_start(const UvPair &p, double dt)
 // relative, a tenth of an FP64 ulp (checked in extended precision against the solved equation
 // on 12000 attractive and repulsive pairs drawn around that boundary), so no Newton
 // correction runs and uv_compose_series composes the half-displacement from S.  Otherwise
-// uv_series_start gives the third-order sum x (1 + c1 + c2) (error O((dt/T)^3), one Newton
-// correction below the 1e-10 acceptance at small steps).  The ALG kernels keep uv_start:
+// uv_series_start gives the start of uv_iterate.  The ALG kernels keep uv_start:
 // changing the code they inline changes how the compiler contracts their own FP64
 // expressions.  Every product and sum is written out (fma, __dmul_rn) so that each kernel
 // that inlines this computes the same bits and takes the same branch: the ensemble's systems
@@ -967,6 +965,7 @@ struct UvSeries {
     double x, y, x2, w, c2;
     double mh;  // -m/2
     double S;   // s = x S where exact
+    double tail;  // c3 + c4
     bool exact;
 };
 
@@ -987,16 +986,20 @@ __device__ __forceinline__ UvSeries uv_series(const UvPair &p, double dt)
     const double c4 = fma(z, fma(3.0, z, __dmul_rn(w, 0.05)), __dmul_rn(y2, fma(14.0, y2, fma(-21.0, z, -0.5 * w))));
     constexpr double Q = 3e-4;
     const bool small = fabs(y) <= Q && fabs(q.c2) <= Q * Q && fabs(c3) <= Q * Q * Q && fabs(c4) <= Q * Q * Q * Q;
-    q.S = 1.0 + (q.c2 - y + (c3 + c4));
+    q.tail = c3 + c4;
+    q.S = 1.0 + (q.c2 - y + q.tail);
     q.exact = small && q.S > 0.0 && dt > 0.0;  // s = x S > 0
     return q;
 }
 
-// The third-order start for a pair whose series is not exact (uv_iterate corrects it).
+// The start for a pair whose series is not exact (uv_iterate corrects it): the fifth-order sum where its last
+// terms are small (at steps a few times the exactness bound its error is ~1e-13 and the first Newton
+// correction is below uv_iterate's acceptance; with the third-order sum it took two: 16384-body Coulomb cube at
+// dt = 1e-3, universal-variable step 3.37 -> 2.95 ms), else the third-order one.
 __device__ __forceinline__ double uv_series_start(const UvSeries &q)
 {
-    const double s3 = __dmul_rn(q.x, 1.0 + (q.c2 - q.y));
-    return (s3 > 0.0) ? s3 : q.x;
+    const double s = __dmul_rn(q.x, fabs(q.tail) <= 0.02 ? q.S : 1.0 + (q.c2 - q.y));
+    return (s > 0.0) ? s : q.x;
 }
 
 // Half-displacement of an exact series pair: the coefficients of uv_compose in the series'
@@ -1057,7 +1060,7 @@ __device__ __forceinline__ int uv_iterate(const UvPair &p, double dt, double &s_
         const double F = p.r0 * s * c[1] + p.sig * s * s * c[2] + p.mu * s * s * s * c[3] - dt;
         const double Fp = p.r0 * c[0] + p.sig * s * c[1] + p.mu * s * s * c[2];
         if (F == 0.0) break;
-        ifp_last = 1.0 / Fp;
+        ifp_last = rcp_normal(Fp);
         const double step = F * ifp_last;
         if (Fp > 0.0 && fabs(step) <= 4.0 * 2.220446049250313e-16 * fabs(s)) {
             s = s - step;  // converged: the remaining correction is a few ulps
@@ -1090,7 +1093,7 @@ __device__ __forceinline__ double uv_halley_step(const UvPair &p, double dt, dou
     const double F = p.r0 * s * c[1] + p.sig * s * s * c[2] + p.mu * s * s * s * c[3] - dt;
     const double Fp = p.r0 * c[0] + p.sig * s * c[1] + p.mu * s * s * c[2];
     const double Fpp = p.sig * c[0] + (p.mu - p.beta * p.r0) * s * c[1];
-    return F * Fp / (Fp * Fp - 0.5 * F * Fpp);
+    return F * Fp * rcp_normal(Fp * Fp - 0.5 * F * Fpp);
 }
 
 // Half-displacement from the solved s: f - 1, g - dt, f', g' - 1 from the Stumpff
@@ -1115,10 +1118,10 @@ __device__ __forceinline__ void uv_compose(const UvPair &p, double s, const doub
             const double x1 = fma(irr_hint, e, irr_hint);
             irr = fma(x1, fma(-rr, x1, 1.0), x1);
         } else {
-            irr = 1.0 / rr;
+            irr = rcp_normal(rr);
         }
     } else {
-        irr = (irr_hint != 0.0 && fabs(e) <= 1e-8) ? fma(irr_hint, e, irr_hint) : 1.0 / rr;
+        irr = (irr_hint != 0.0 && fabs(e) <= 1e-8) ? fma(irr_hint, e, irr_hint) : rcp_normal(rr);
     }
     // the half-displacement's factor 1/2 is taken into the coefficients: scaling by a power of
     // two is exact, so h is the same as (f - 1) r + (g - dt) v halved afterwards, at four

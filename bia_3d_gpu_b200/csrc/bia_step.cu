@@ -374,8 +374,11 @@ __global__ void __launch_bounds__(kMlpThreads, 2) bia_pair_learned_kernel(const 
 // Split learned step, second kernel: the rows of both heads on the tensor cores (persistent
 // CTAs of kMlpThreads, TMEM allocated once per CTA).  A timed-out pipeline is counted; its
 // rows keep their inputs, which the finish kernel's FP64 step rejects (the plain solver
-// takes those pairs).
-__global__ void __launch_bounds__(kMlpThreads, 2) bia_pair_learned_head_kernel(const LearnedRows R,
+// takes those pairs).  Four CTAs per SM (all of the tensor memory, 512 of its columns, and 214 KB of shared
+// memory): a 256-row tile is a chain of three MMAs and epilogues, 9400 cycles at two CTAs.  6e7 rows (Coulomb
+// cube, n = 16384, dt = 1e-3): 3.87 ms at two, 3.46 at four.
+constexpr int kHeadCtas = 4;
+__global__ void __launch_bounds__(kMlpThreads, kHeadCtas) bia_pair_learned_head_kernel(const LearnedRows R,
                                                                                  const MlpImage *heads,
                                                                                  unsigned long long *stats)
 {
@@ -510,9 +513,9 @@ static int learned_kernel_setup()
         ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bia_pair_learned_head_kernel, kMlpThreads,
                                                                  (size_t)hbytes) == cudaSuccess;
         if (!ok) cudaGetLastError();
-        // at least the launch bound's two CTAs per SM: CTAs beyond the resident ones wait
+        // at least the launch bound's CTAs per SM: CTAs beyond the resident ones wait
         // for a slot, so a low answer costs nothing but a short queue
-        grid_of[dev] = ok ? sms * (occ > 2 ? occ : 2) : 0;
+        grid_of[dev] = ok ? sms * (occ > kHeadCtas ? occ : kHeadCtas) : 0;
         done_of[dev] = true;
     }
     return grid_of[dev];

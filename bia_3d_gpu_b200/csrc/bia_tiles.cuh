@@ -90,6 +90,16 @@ __device__ __forceinline__ void flush_counters(const PairCounters &c, unsigned l
 constexpr int kTileWarps = 8;              // warps per CTA of every kernel using warp-blocks
 constexpr int kTileSmemDoubles = 13 * 32;  // per warp: column state [7][32], sums [6][32]
 
+// position of the n-th set bit of m (n from 0, below popc(m)), by bisection: __fns walks the bits
+__device__ __forceinline__ int nth_set(unsigned m, int n)
+{
+    int pos = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+        if (__popc(m & ((1u << (pos + step)) - 1u)) <= n) pos += step;
+    return pos;
+}
+
 template <int C>
 __device__ __forceinline__ void compact_class_loop(unsigned m, const double si[7], const double *ws,
                                                    double *wacc, int lane, bool has_q, double eps_th,
@@ -179,7 +189,7 @@ __device__ __forceinline__ void balanced_class_loop(unsigned m, const double *rs
                 const int nr = __popc(rm);
                 const int idx = q - rbase;
                 const bool here = idx >= 0 && idx < nr;
-                const int src = here ? (int)__fns(rm, 0, idx + 1) : 0;
+                const int src = here ? nth_set(rm, idx) : 0;
                 const int kk = __shfl_sync(full, __ffs(cur) - 1, src);  // the owner's pair of this round
                 if (here) {
                     o = src;
