@@ -38,7 +38,7 @@ def _host_f64(a, n, name):
         raise TypeError(f"{name} must be a C-contiguous float64 numpy array")
     if a.size < n:
         raise ValueError(f"{name} has {a.size} elements, need {n}")
-    return a.ctypes.data_as(_PD)
+    return a.ctypes.data
 
 
 def find_dxyuv_kernel(METHOD, N, I, EPS, DT, ITR, dX, dY, dZ, dU, dV, dW, RXYZUVW, dXYZUVW):

@@ -133,9 +133,9 @@ def lib():
     L.rkf_c_.argtypes = [_I, _D, _PD, _PD, _PD, _PI, _PD, _PD, _PD, _PD, _PI, _PI, _PD, _PD, _PD,
                          _PD, _PD]
     L.rkf_c_.restype = None
-    L.find_dxyuv_kernel_.argtypes = [_I, _I, _I, _D, _D, _I] + [_PD] * 8
+    L.find_dxyuv_kernel_.argtypes = [_I, _I, _I, _D, _D, _I] + [_V] * 8
     L.find_dxyuv_kernel_.restype = None
-    L.invariance_gpu_.argtypes = [_I, _D] + [_PD] * 6 + [_PD] * 11
+    L.invariance_gpu_.argtypes = [_I, _D] + [_V] * 6 + [_PD] * 11
     L.invariance_gpu_.restype = None
     _PF = ctypes.POINTER(ctypes.c_float)
     L.bia_trainer_create.argtypes = [_V, _I, ctypes.c_longlong, ctypes.c_ulonglong, ctypes.POINTER(_V)]
