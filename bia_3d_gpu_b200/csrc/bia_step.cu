@@ -153,16 +153,69 @@ __global__ void __launch_bounds__(kW * 32, kMinB) bia_pair_phase_kernel(const St
     if (warp == 0) flush_slots(slots, kW, A.stats, lane);
 }
 
+// ALG, a CTA per warp-block (alg_block_solve): small systems, where a warp per warp-block leaves
+// most of the chip idle and a step lasts as long as one warp's 32 turns of a solver.  What is left is
+// a CTA's chain (four turns, the sums) when there are few blocks, else the FP64 pipes.  Three CTAs
+// of 8 warps per SM (85 registers; their 62 KB of h and states leave L1 enough for the spills) let
+// one's sums overlap another's solves: gravity ball of 1332, 82 us a step against 88 with two CTAs
+// (128 registers, no spills), 94 and 111 with 16-warp CTAs, two and one per SM, and 137 with
+// bia_pair_tiles_kernel; of 257, 34 against 32, 31, 28 and 137; Coulomb cube of 1332, 123 against
+// 132, 141, 185 and 219.
+template <bool kDeterministic>
+__global__ void __launch_bounds__(kBlockWarps * 32, 3) bia_pair_block_kernel(const StepArgs A)
+{
+    extern __shared__ double block_smem[];
+    AlgBlockShared &S = *reinterpret_cast<AlgBlockShared *>(block_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane < kNumStats) S.slots[warp * kNumStats + lane] = 0ull;
+    int bi, bj;
+    warp_block_coords(A.t0 + blockIdx.x, bi, bj);
+    double rsum, csum;
+    PairCounters cnt;
+    counters_zero(cnt);
+    alg_block_solve(A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, A.eps_th, A.P, bi, bj, S, rsum, csum, cnt);
+    counters_to_slot(cnt, S.slots + warp * kNumStats, lane);
+    if (warp < 6) {
+        const size_t plane = (size_t)A.npad;
+        const int i = bi * 32 + lane, j = bj * 32 + lane;
+        if (kDeterministic) {
+            if (bi == bj) {
+                A.part[((size_t)bi * 6 + warp) * plane + i] = rsum - csum;
+            } else {
+                A.part[((size_t)bj * 6 + warp) * plane + i] = rsum;
+                A.part[((size_t)bi * 6 + warp) * plane + j] = -csum;
+            }
+        } else if (bi == bj) {
+            if (i < A.n) atomicAdd(&A.part[warp * plane + i], rsum - csum);
+        } else {
+            if (i < A.n) atomicAdd(&A.part[warp * plane + i], rsum);
+            if (j < A.n) atomicAdd(&A.part[warp * plane + j], -csum);
+        }
+    }
+    __syncthreads();
+    if (warp == 0) flush_slots(S.slots, kBlockWarps, A.stats, lane);
+}
+
 // ALG pair-kernel shapes the autotuner chooses from (bia_context_autotune):
-//   kVarTiles8    8-warp CTAs, per-warp class phases (bia_pair_tiles_kernel)
+//   kVarTiles8    8-warp CTAs, per-warp class phases (bia_pair_tiles_kernel), below
+//                 kBlockMaxPerSm warp-blocks per SM a CTA per warp-block (bia_pair_block_kernel)
 //   kVarPhase32Lane phase-locked CTAs of 32 warps, 1 per SM, per-lane class loops (rows in
 //                 registers: all-hyperbolic systems, where packing saves no turn)
 //   kVarPhase32   phase-locked CTAs of 32 warps, 1 per SM (64 registers), balanced class
 //                 loops (mixed classes)
-// (CTAs of 16 warps, 2 per SM, were never the fastest: Plummer 72.6, Coulomb 111 ms against
-// 70.9 and 82.7 ms for kVarPhase32 at n = 32768.)  All shapes give bitwise the same step.
-// Without a tuned entry the step takes kVarPhase32 when it gives at least two CTAs per SM,
-// else kVarTiles8.
+// All shapes give bitwise the same step.  Measured, us a step (gravity ball, hyperbolic | Coulomb
+// cube, mixed):
+//   n       warp-blocks/SM   block          tiles          phase32
+//   1332        6.1           99 |  137     144 |  223     300 |  387
+//   2000       13.6          169 |  281     184 |  301     300 |  391
+//   3000       30.2          323 |  591     339 |  632     306 |  404
+//   4300       62.0          602 | 1191     585 | 1201     583 |  768
+//   10000      331          3016 | 6321    2764 | 6866    3038 | 4022
+// A phase32 wave lasts the same however many of its 32 warps per SM have a block, so it is taken
+// from three quarters of a wave on (between the points where the two systems change over), up to a
+// full one, and again from three quarters of the second on; between and below, the block kernel.
+// A pinned kVarTiles8 changes to tiles at that last point, the hyperbolic systems' crossing.
+constexpr long long kPhaseMinPerSm = 24, kBlockMaxPerSm = 48;
 enum AlgVariant { kVarTiles8 = 0, kVarPhase32Lane = 1, kVarPhase32 = 2, kVarCount = 3 };
 
 // the warps' slices, then one counter slot of kNumStats u64 per warp
@@ -195,6 +248,10 @@ static int phase_kernel_setup()
                                         phase_smem_bytes<32, false>()) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(bia_pair_phase_kernel<false, 32, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         phase_smem_bytes<32, false>()) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(AlgBlockShared)) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(AlgBlockShared)) == cudaSuccess;
         if (!ok) cudaGetLastError();  // clear; the 8-warp kernel is used instead
         sms_of[dev] = ok ? sms : 0;
         done_of[dev] = true;
@@ -209,7 +266,8 @@ static int alg_variant_for(long long nwb, int tuned)
     const int sms = phase_kernel_setup();
     if (sms <= 0 || BIA_PHASE_WARPS == 0) return kVarTiles8;
     if (tuned >= 0 && tuned < kVarCount) return tuned;
-    return ((nwb + 31) / 32 >= 2LL * sms) ? kVarPhase32 : kVarTiles8;
+    const bool one_wave = nwb >= kPhaseMinPerSm * sms && nwb <= 32LL * sms;
+    return one_wave || nwb >= kBlockMaxPerSm * sms ? kVarPhase32 : kVarTiles8;
 }
 
 // CTAs per SM of the persistent universal-variable and rest kernels (their launch bound)
@@ -297,6 +355,11 @@ static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st
         if (var == kVarPhase32Lane) {
             bia_pair_phase_kernel<kDeterministic, 32, 1, false>
                 <<<(unsigned)((A.nwb + 31) / 32), 32 * 32, phase_smem_bytes<32, false>(), st>>>(A);
+            return;
+        }
+        if (var == kVarTiles8 && A.nwb < kBlockMaxPerSm * phase_kernel_setup()) {
+            bia_pair_block_kernel<kDeterministic>
+                <<<(unsigned)A.nwb, kBlockWarps * 32, sizeof(AlgBlockShared), st>>>(A);
             return;
         }
     }

@@ -388,6 +388,151 @@ __device__ __forceinline__ void phase_block_solve(const double *x, const double 
     }
 }
 
+// One warp-block solved by a CTA's warps together (ALG).  The classes' pairs are listed, each
+// class from a multiple of 32 on, and the warps take the list in steps of 32: a warp's turn is one
+// class, as in the loops above, and a block takes ceil(turns / warps) of a turn's time.  Each pair's
+// h waits in shared memory; then a warp per component adds the rows and the columns in the loops'
+// order (a row its pairs of a class in bit order; a column by the pair's rank in its row, then by
+// row), so the sums are bitwise theirs.
+constexpr int kBlockWarps = 8;
+struct AlgBlockShared {
+    double h[6][32 * 32];              // [component][32 k + row]: the pair of row and column (row + k) mod 32
+    double row[7][32], col[7][32];
+    unsigned long long slots[kBlockWarps * kNumStats];
+    unsigned mask[3][32];              // per class and row: bit k
+    unsigned count[3][32];             // per class and k: pairs
+    unsigned at_rank[32][32];          // per rank and column: the rows
+    unsigned short list[32 * 32 + 64];
+};
+
+// every thread of the CTA calls it; warps c < 6 get component c's sums of row and column `lane`
+__device__ __forceinline__ void alg_block_solve(const double *x, const double *y, const double *z, const double *u,
+                                                const double *v, const double *w, const double *q, int n,
+                                                double eps_th, const PairParams &P, int bi, int bj, AlgBlockShared &S,
+                                                double &rsum, double &csum, PairCounters &cnt)
+{
+    const unsigned full = 0xffffffffu;
+    constexpr int kTurns = 32 / kBlockWarps;  // values of k a warp classifies
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool diag = bi == bj, has_q = q != nullptr;
+    const int i = bi * 32 + lane;
+    if (warp < 2) {
+        double s[7];
+        load_particle(x, y, z, u, v, w, q, n, (warp ? bj : bi) * 32 + lane, s);
+#pragma unroll
+        for (int c = 0; c < 7; c++) (warp ? S.col : S.row)[c][lane] = s[c];
+    } else if (warp < 5) {
+        S.mask[warp - 2][lane] = 0u;
+    }
+    __syncthreads();
+    int cls[kTurns], pos[kTurns];
+#pragma unroll
+    for (int t = 0; t < kTurns; t++) {
+        const int k = warp * kTurns + t, src = (lane + k) & 31;
+        const bool ok = i < n && bj * 32 + src < n && (!diag || (k > 0 && (k < 16 || (k == 16 && lane < 16))));
+        cls[t] = 3;
+        if (ok) {
+            const double r[3] = {S.row[0][lane] - S.col[0][src], S.row[1][lane] - S.col[1][src], S.row[2][lane] - S.col[2][src]};
+            const double g[3] = {S.row[3][lane] - S.col[3][src], S.row[4][lane] - S.col[4][src], S.row[5][lane] - S.col[5][src]};
+            const double eps_ij = has_q ? eps_th * S.row[6][lane] * S.col[6][src] : eps_th;
+            const int c = alg_classify(eps_ij, r, g);
+            cls[t] = c == kClsHyp ? 0 : c == kClsEll ? 1 : 2;
+            atomicOr(&S.mask[cls[t]][lane], 1u << k);
+        }
+        __syncwarp();
+        pos[t] = 0;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const unsigned b = __ballot_sync(full, cls[t] == c);
+            if (lane == 0) S.count[c][k] = __popc(b);
+            if (cls[t] == c) pos[t] = __popc(b & ((1u << lane) - 1u));
+        }
+    }
+    __syncthreads();
+    // pairs of each class with a smaller k (lane = k), 16 bits a class
+    unsigned long long own = 0ull, upto;
+#pragma unroll
+    for (int c = 0; c < 3; c++) own |= (unsigned long long)S.count[c][lane] << (16 * c);
+    upto = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long o = __shfl_up_sync(full, upto, off);
+        if (lane >= off) upto += o;
+    }
+    const unsigned long long all = __shfl_sync(full, upto, 31);
+    const int nh = (int)(all & 0xffff), ne = (int)(all >> 16 & 0xffff), nr = (int)(all >> 32 & 0xffff);
+    const int e0 = (nh + 31) & ~31, r0 = e0 + ((ne + 31) & ~31), end = r0 + nr;
+    upto -= own;
+#pragma unroll
+    for (int t = 0; t < kTurns; t++) {
+        const unsigned long long before = __shfl_sync(full, upto, warp * kTurns + t);
+        if (cls[t] < 3) {
+            const int at = (cls[t] == 0 ? 0 : cls[t] == 1 ? e0 : r0) + (int)(before >> (16 * cls[t]) & 0xffff) + pos[t];
+            S.list[at] = (unsigned short)((warp * kTurns + t) * 32 + lane);
+        }
+    }
+    __syncthreads();
+    for (int s = warp * 32; s < end; s += 32 * kBlockWarps) {
+        const int c = s < e0 ? 0 : s < r0 ? 1 : 2;
+        if (s + lane < (c == 0 ? nh : c == 1 ? e0 + ne : end)) {
+            const int id = S.list[s + lane];
+            const int o = id & 31, j = (o + (id >> 5)) & 31;
+            double si[7], sc[7];
+#pragma unroll
+            for (int m = 0; m < 7; m++) {
+                si[m] = S.row[m][o];
+                sc[m] = S.col[m][j];
+            }
+            const double r[3] = {si[0] - sc[0], si[1] - sc[1], si[2] - sc[2]};
+            const double g[3] = {si[3] - sc[3], si[4] - sc[4], si[5] - sc[5]};
+            const double eps_ij = has_q ? eps_th * si[6] * sc[6] : eps_th;
+            double h[6];
+            if (c == 0) alg_conic_pair<kClsHyp>(P, eps_ij, r, g, h, cnt);
+            else if (c == 1) alg_conic_pair<kClsEll>(P, eps_ij, r, g, h, cnt);
+            else alg_rare_pair(P, eps_ij, r, g, h, cnt, alg_classify(eps_ij, r, g));
+#pragma unroll
+            for (int m = 0; m < 6; m++) S.h[m][id] = h[m];
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    rsum = csum = 0.0;
+    const double *h = S.h[warp < 6 ? warp : 0];
+    for (int c = 0; c < 3; c++) {  // block-uniform
+        const unsigned m = S.mask[c][lane];
+        const int most = (int)__reduce_max_sync(full, (unsigned)__popc(m));
+        if (most == 0) continue;
+        if (__all_sync(full, m == full)) {  // rank k of every row is its pair k
+            if (warp < 6) {
+#pragma unroll 8
+                for (int k = 0; k < 32; k++) {
+                    rsum += h[32 * k + lane];
+                    csum += h[32 * k + ((lane - k) & 31)];
+                }
+            }
+            continue;
+        }
+#pragma unroll
+        for (int t = 0; t < kTurns; t++) S.at_rank[warp * kTurns + t][lane] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < kTurns; t++) {
+            const int k = warp * kTurns + t;
+            if (m >> k & 1u) atomicOr(&S.at_rank[__popc(m & ((1u << k) - 1u))][(lane + k) & 31], 1u << lane);
+        }
+        __syncthreads();
+        if (warp < 6) {
+            for (unsigned left = m; left; left &= left - 1u) rsum += h[32 * (__ffs(left) - 1) + lane];
+            for (int r = 0; r < most; r++)
+                for (unsigned rows = S.at_rank[r][lane]; rows; rows &= rows - 1u) {
+                    const int o = __ffs(rows) - 1;
+                    csum += h[32 * ((lane - o) & 31) + o];
+                }
+        }
+        __syncthreads();
+    }
+}
+
 constexpr size_t kSliceBytes = kTileWarps * kTileSmemDoubles * sizeof(double);
 
 // The column slice of the universal-variable, rest and RKF45 walks: the column states as three
