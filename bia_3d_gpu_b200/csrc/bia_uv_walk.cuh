@@ -28,8 +28,9 @@ namespace bia {
 // different slot on every lane), and leaves a bit for every other pair (bit k of the returned
 // mask).  Full off-diagonal blocks take two offsets a turn without a test of their particles: the
 // branch-free pairs of two offsets interleave, where one pair's chain of dependent FP64 operations
-// alone left the warp waiting.  A block whose first kProbe offsets hold mostly other pairs (a
-// long step) leaves the rest of them to the second pass untried.
+// alone left the warp waiting.  A block more than a quarter of whose first kProbe offsets' pairs are
+// others (a long step) leaves the rest of them to the second pass untried: 7.63 ms against 8.07 at
+// a half and 7.63 at an eighth (learned, Coulomb, n = 16384, 1e-4), where half of the pairs are others.
 //
 // Out of line, on the dynamic shared memory of the kernel (the warp's slice begins `slice` doubles
 // into it), so that the loop has the whole register budget whatever the kernel around it keeps:
@@ -71,7 +72,7 @@ static __device__ __noinline__ unsigned uv_walk_full(int slice, const UvRow row,
             slice_add(ws, src[u], h[u], racc);
             __syncwarp();  // slot src is the next offset's slot of lane - 1
         }
-        if (k + 2 == kProbe && __reduce_add_sync(0xffffffffu, (unsigned)__popc(left)) > 32u * kProbe / 2u) {
+        if (k + 2 == kProbe && __reduce_add_sync(0xffffffffu, (unsigned)__popc(left)) > 32u * kProbe / 4u) {
             left |= 0xffffffffu << kProbe;
             break;
         }
@@ -111,14 +112,19 @@ static __device__ __noinline__ unsigned uv_walk_part(int slice, const UvRow row,
 // The second pass: slow(src, k, h) gives h of the pairs in `left`, in ascending k on each lane.  Few
 // of them: every lane takes its own next one each turn, so a turn solves a pair on as many lanes
 // as have one left, and lanes that meet in a column add in lane order.  Many: the lanes walk the
-// offsets together (distinct columns).  Which, depends on the block's pairs alone.
+// offsets together (distinct columns).  Which, depends on the block's pairs alone.  The line at half
+// of the block's pairs: Plummer, n = 16384, a universal-variable step of 1e-3, 3.46 ms at a quarter,
+// 3.40 at half, 3.56 at three quarters; the Coulomb cubes there differ by 1 %.  The universal-variable
+// solve is in line in both loops: 2.80 against 3.56 ms out of line (Coulomb, 1e-4), 1.5 % slower
+// where the walk leaves few pairs; the rest pass's pair, longer, is faster out of line (13.05
+// against 13.65 ms for the learned step of 1e-3).
 template <class Slow>
 __device__ __forceinline__ void uv_walk_rest(unsigned left, double *ws, int lane, const double si[7], double racc[6],
                                              Slow &slow)
 {
     const unsigned full = 0xffffffffu;
     const unsigned count = __reduce_add_sync(full, (unsigned)__popc(left));
-    if (count <= 256u) {
+    if (count <= 512u) {
         const unsigned lt = (1u << lane) - 1u;
         for (;;) {
             const bool busy = left != 0u;
@@ -164,16 +170,6 @@ __device__ __forceinline__ int block_lane_pairs(int lane, int bi, int bj, int n)
     for (int k = 1; k <= 16; k++) c += ((k < 16 || lane < 16) && ((lane + k) & 31) < ncols) ? 1 : 0;
     return c;
 }
-
-// The universal-variable pair that is not a short-step one, out of line: one body for every
-// kernel of a file, so that all compute the same bits, and a small walk.
-static __device__ __noinline__ int uv_slow_pair(double eps_ij, double dt, double rx, double ry, double rz, double gx,
-                                                double gy, double gz, double *h)
-{
-    const double r[3] = {rx, ry, rz}, g[3] = {gx, gy, gz};
-    return uv_halfdisp_fast(eps_ij, dt, r, g, h);
-}
-
 
 // A system as the walk sees it: particles x..w[0, n) (charges q), coupling eps_th, and where its
 // partial sums go (deterministic: part[m][6][plane]; atomic: one accumulator plane).
@@ -225,7 +221,7 @@ __device__ __forceinline__ int walk_other_pair(double eps_ij, double dt, const d
             return kind;
         }
     } else {
-        it = uv_slow_pair(eps_ij, dt, r[0], r[1], r[2], g[0], g[1], g[2], hs);
+        it = uv_halfdisp_fast(eps_ij, dt, r, g, hs);  // in line: see uv_walk_rest
     }
     bool finite = true;
 #pragma unroll
