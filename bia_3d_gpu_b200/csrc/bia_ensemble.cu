@@ -454,7 +454,7 @@ static int ens_pair_launch(bia_context *ctx, bia_ensemble *E, EnsArgs &A, int me
                                       walk_smem_bytes<false>(kEnsWarps), st>>>(A);
         break;
     default: {
-        const int sms = BIA_PHASE_WARPS > 0 ? ens_phase_setup() : 0;
+        const int sms = ens_phase_setup();
         int var = shape;
         if (var < 0 || var >= kEnsShapes) var = (sms > 0 && (E->nitems + 31) / 32 >= 2LL * sms) ? 2 : 0;
         if (sms <= 0) var = 0;

@@ -58,12 +58,12 @@ struct StepArgs {
     LearnedRows R;
 };
 
-// ALG and RKF45: each warp solves warp-blocks t = (its global warp index) + k * (warps in the grid), one
+// ALG: each warp solves warp-blocks t = (its global warp index) + k * (warps in the grid), one
 // block per warp when the grid covers every block.  The counters are summed per warp in
 // registers and flushed every kFlushBlocks blocks: one set of atomics per warp instead of one
 // per block.
-template <bool kDeterministic, int M>
-__global__ void __launch_bounds__(kThreads, TileOccupancy<M>::kMinBlocks) bia_pair_tiles_kernel(const StepArgs A)
+template <bool kDeterministic>
+__global__ void __launch_bounds__(kThreads, TileOccupancy<kMethodAlg>::kMinBlocks) bia_pair_tiles_kernel(const StepArgs A)
 {
     const int lane = threadIdx.x & 31;
     PairCounters tot;
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kThreads, TileOccupancy<M>::kMinBlocks) bia_pa
         const bool diag = (bi == bj);
         double racc[6], cacc[6];
         PairCounters cnt;
-        warp_block_solve<M>(A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, A.eps_th, A.P, bi, bj, lane, racc, cacc, cnt);
+        warp_block_solve<kMethodAlg>(A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, A.eps_th, A.P, bi, bj, lane, racc, cacc, cnt);
         counters_add(tot, cnt);
         if (++nblk == kFlushBlocks) {
             flush_counters(tot, A.stats, lane);
@@ -153,6 +153,27 @@ __global__ void __launch_bounds__(kW * 32, kMinB) bia_pair_phase_kernel(const St
     if (warp == 0) flush_slots(slots, kW, A.stats, lane);
 }
 
+// component c's sums of row and column `lane` of a warp-block onto the partials or accumulators
+template <bool kDeterministic>
+__device__ __forceinline__ void block_write(const StepArgs &A, int bi, int bj, int c, int lane, double rsum, double csum)
+{
+    const size_t plane = (size_t)A.npad;
+    const int i = bi * 32 + lane, j = bj * 32 + lane;
+    if (kDeterministic) {
+        if (bi == bj) {
+            A.part[((size_t)bi * 6 + c) * plane + i] = rsum - csum;
+        } else {
+            A.part[((size_t)bj * 6 + c) * plane + i] = rsum;
+            A.part[((size_t)bi * 6 + c) * plane + j] = -csum;
+        }
+    } else if (bi == bj) {
+        if (i < A.n) atomicAdd(&A.part[c * plane + i], rsum - csum);
+    } else {
+        if (i < A.n) atomicAdd(&A.part[c * plane + i], rsum);
+        if (j < A.n) atomicAdd(&A.part[c * plane + j], -csum);
+    }
+}
+
 // ALG, a CTA per warp-block (alg_block_solve): small systems, where a warp per warp-block leaves
 // most of the chip idle and a step lasts as long as one warp's 32 turns of a solver.  What is left is
 // a CTA's chain (four turns, the sums) when there are few blocks, else the FP64 pipes.  Three CTAs
@@ -175,25 +196,77 @@ __global__ void __launch_bounds__(kBlockWarps * 32, 3) bia_pair_block_kernel(con
     counters_zero(cnt);
     alg_block_solve(A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, A.eps_th, A.P, bi, bj, S, rsum, csum, cnt);
     counters_to_slot(cnt, S.slots + warp * kNumStats, lane);
-    if (warp < 6) {
-        const size_t plane = (size_t)A.npad;
-        const int i = bi * 32 + lane, j = bj * 32 + lane;
-        if (kDeterministic) {
-            if (bi == bj) {
-                A.part[((size_t)bi * 6 + warp) * plane + i] = rsum - csum;
-            } else {
-                A.part[((size_t)bj * 6 + warp) * plane + i] = rsum;
-                A.part[((size_t)bi * 6 + warp) * plane + j] = -csum;
-            }
-        } else if (bi == bj) {
-            if (i < A.n) atomicAdd(&A.part[warp * plane + i], rsum - csum);
-        } else {
-            if (i < A.n) atomicAdd(&A.part[warp * plane + i], rsum);
-            if (j < A.n) atomicAdd(&A.part[warp * plane + j], -csum);
-        }
-    }
+    if (warp < 6) block_write<kDeterministic>(A, bi, bj, warp, lane, rsum, csum);
     __syncthreads();
     if (warp == 0) flush_slots(S.slots, kBlockWarps, A.stats, lane);
+}
+
+// RKF45, a CTA per warp-block: each warp integrates four of its rotation offsets, every h waits in
+// shared memory, and a warp per component adds the rows and the columns in the offsets' order (the
+// sums of warp_block_solve_rkf, bitwise).  A warp per warp-block, before, made a small step last as
+// long as 32 integrations and gave a few hard pairs the time of their whole warp-block.  Bound by
+// the FP64 pipes from about 900 warp-blocks on, by a CTA's four integrations below.  Two CTAs per SM
+// (128 registers, 53 KB).  Measured, us a step, Plummer sphere of 257, 1332, 3000, 8191: 61, 200, 782,
+// 5481, against 292, 305, 861, 5637; Coulomb cube: 67, 349, 803, 5624, against 299, 502, 932, 5744.
+struct RkfBlockShared {
+    double h[6][32 * 32];  // [component][32 k + row], as AlgBlockShared's
+    double row[7][32], col[7][32];
+    unsigned long long slots[kBlockWarps * kNumStats];
+};
+
+template <bool kDeterministic>
+__global__ void __launch_bounds__(kBlockWarps * 32, 2) bia_pair_block_rkf_kernel(const StepArgs A)
+{
+    extern __shared__ double block_smem[];
+    RkfBlockShared &S = *reinterpret_cast<RkfBlockShared *>(block_smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool has_q = A.q != nullptr;
+    for (long long t = blockIdx.x; t < A.nwb; t += gridDim.x) {  // one turn unless the grid's limit is below nwb
+        int bi, bj;
+        warp_block_coords(A.t0 + t, bi, bj);
+        const bool diag = bi == bj;
+        const int i = bi * 32 + lane, j = bj * 32 + lane;
+        if (lane < kNumStats) S.slots[warp * kNumStats + lane] = 0ull;
+        if (warp < 2) {
+            double s[7];
+            load_particle(A.x, A.y, A.z, A.u, A.v, A.w, A.q, A.n, warp ? j : i, s);
+#pragma unroll
+            for (int c = 0; c < 7; c++) (warp ? S.col : S.row)[c][lane] = s[c];
+        }
+        __syncthreads();
+        const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
+        PairCounters cnt;
+        counters_zero(cnt);
+        for (int k = k0 + warp; k <= k1; k += kBlockWarps) {
+            const int src = (lane + k) & 31;
+            double h[6] = {0, 0, 0, 0, 0, 0};
+            if ((!diag || k < 16 || lane < 16) && i < A.n && bj * 32 + src < A.n) {
+                const double r[3] = {S.row[0][lane] - S.col[0][src], S.row[1][lane] - S.col[1][src],
+                                     S.row[2][lane] - S.col[2][src]};
+                const double g[3] = {S.row[3][lane] - S.col[3][src], S.row[4][lane] - S.col[4][src],
+                                     S.row[5][lane] - S.col[5][src]};
+                const double eps_ij = has_q ? A.eps_th * S.row[6][lane] * S.col[6][src] : A.eps_th;
+                pair_halfdisp<kMethodRkf>(A.P, eps_ij, r, g, h, cnt);
+            }
+#pragma unroll
+            for (int c = 0; c < 6; c++) S.h[c][32 * k + lane] = h[c];
+        }
+        counters_to_slot(cnt, S.slots + warp * kNumStats, lane);
+        __syncthreads();
+        if (warp < 6) {
+            double rsum = 0.0, csum = 0.0;
+            const double *h = S.h[warp];
+#pragma unroll 8
+            for (int k = k0; k <= k1; k++) {
+                rsum += h[32 * k + lane];
+                csum += h[32 * k + ((lane - k) & 31)];
+            }
+            block_write<kDeterministic>(A, bi, bj, warp, lane, rsum, csum);
+        } else if (warp == 6) {
+            flush_slots(S.slots, kBlockWarps, A.stats, lane);
+        }
+        __syncthreads();
+    }
 }
 
 // ALG pair-kernel shapes the autotuner chooses from (bia_context_autotune):
@@ -252,6 +325,10 @@ static int phase_kernel_setup()
                                         (int)sizeof(AlgBlockShared)) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(bia_pair_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sizeof(AlgBlockShared)) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_block_rkf_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(RkfBlockShared)) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_block_rkf_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(RkfBlockShared)) == cudaSuccess;
         if (!ok) cudaGetLastError();  // clear; the 8-warp kernel is used instead
         sms_of[dev] = ok ? sms : 0;
         done_of[dev] = true;
@@ -264,7 +341,7 @@ static int phase_kernel_setup()
 static int alg_variant_for(long long nwb, int tuned)
 {
     const int sms = phase_kernel_setup();
-    if (sms <= 0 || BIA_PHASE_WARPS == 0) return kVarTiles8;
+    if (sms <= 0) return kVarTiles8;
     if (tuned >= 0 && tuned < kVarCount) return tuned;
     const bool one_wave = nwb >= kPhaseMinPerSm * sms && nwb <= 32LL * sms;
     return one_wave || nwb >= kBlockMaxPerSm * sms ? kVarPhase32 : kVarTiles8;
@@ -365,14 +442,16 @@ static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st
     }
     switch (A.P.method) {
     case kMethodRkf:
-        bia_pair_tiles_kernel<kDeterministic, kMethodRkf><<<(unsigned)grid, kThreads, kSliceBytes, st>>>(A);
+        phase_kernel_setup();
+        bia_pair_block_rkf_kernel<kDeterministic>
+            <<<(unsigned)(A.nwb < 0x7fffffffLL ? A.nwb : 0x7fffffffLL), kBlockWarps * 32, sizeof(RkfBlockShared), st>>>(A);
         break;
     case kMethodUniversal:
         bia_pair_walk_kernel<kDeterministic, false>
             <<<(unsigned)persistent_grid(grid), kThreads, walk_smem_bytes<false>(kWarpsPerBlock), st>>>(A);
         break;
     default:
-        bia_pair_tiles_kernel<kDeterministic, kMethodAlg><<<(unsigned)grid, kThreads, 0, st>>>(A);
+        bia_pair_tiles_kernel<kDeterministic><<<(unsigned)grid, kThreads, 0, st>>>(A);
         break;
     }
 }

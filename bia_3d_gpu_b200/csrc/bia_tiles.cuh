@@ -1,13 +1,11 @@
 // bia_tiles.cuh -- one 32 x 32 warp-block of pairs, shared by the single-system step
 // (bia_step.cu) and the ensemble step (bia_ensemble.cu).
 //
-// Lane l keeps row particle 32*bi + l and column particle 32*bj + l in registers.  At
-// rotation step k it solves the pair (row l, column (l + k) mod 32), the column state
-// arriving by shuffle, and the column's half-displacement goes back by a second shuffle
-// from lane (l - k) mod 32, so every lane works on a different pair and both sums stay in
-// registers.  Off-diagonal blocks take 32 steps (1024 pairs); diagonal blocks 16 (k =
-// 1..15 on all lanes, k = 16 on lanes 0..15: each of the 496 pairs once; orientation does
-// not matter because the half-displacement is exactly antisymmetric under i <-> j).
+// Lane l owns row particle 32*bi + l; the column particles and their sums lie in shared memory.  At
+// rotation offset k it solves the pair (row l, column (l + k) mod 32), so every lane works on a
+// different pair and adds to a different column.  Off-diagonal blocks have 32 offsets (1024 pairs);
+// diagonal blocks 16 (k = 1..15 on all lanes, k = 16 on lanes 0..15: each of the 496 pairs once;
+// orientation does not matter because the half-displacement is exactly antisymmetric under i <-> j).
 #pragma once
 #include <mutex>
 
@@ -19,22 +17,9 @@ namespace bia {
 // Resident CTAs per SM each method's 8-warp kernel is compiled for (register budget
 // 65536 / (256 threads * blocks)): ALG 3 (<= 85 registers, measured fastest on the
 // mixed-class Coulomb workload) and RKF45 2 (<= 128).
-#ifndef BIA_ALG_MIN_BLOCKS
-#define BIA_ALG_MIN_BLOCKS 3
-#endif
-// RKF45: the shared-memory column walk at two CTAs per SM (128 registers; 270 B of spills
-// around the out-of-line pair integrator) measured 184 ms per Coulomb step at n = 32768
-// against 245 ms for the shuffle walk at one CTA per SM (222 registers) and 194 ms for the
-// shuffle walk at two; bitwise the same sums.
-#ifndef BIA_RKF_MIN_BLOCKS
-#define BIA_RKF_MIN_BLOCKS 2
-#endif
-#ifndef BIA_RKF_SMEM
-#define BIA_RKF_SMEM 1  // RKF walks with the column slice in shared memory
-#endif
 template <int M> struct TileOccupancy { static constexpr int kMinBlocks = 1; };
-template <> struct TileOccupancy<kMethodRkf> { static constexpr int kMinBlocks = BIA_RKF_MIN_BLOCKS; };
-template <> struct TileOccupancy<kMethodAlg> { static constexpr int kMinBlocks = BIA_ALG_MIN_BLOCKS; };
+template <> struct TileOccupancy<kMethodRkf> { static constexpr int kMinBlocks = 2; };
+template <> struct TileOccupancy<kMethodAlg> { static constexpr int kMinBlocks = 3; };
 
 __device__ __forceinline__ void warp_block_coords(long long t, int &bi, int &bj)
 {
@@ -84,9 +69,6 @@ __device__ __forceinline__ void flush_counters(const PairCounters &c, unsigned l
 // column sums live in this warp's slice of shared memory; lanes that hit the same column
 // in one turn add their h in lane order (__match_any_sync groups), so the column sums
 // have a fixed order for given inputs and the step stays bitwise reproducible.
-#ifndef BIA_ALG_COMPACT
-#define BIA_ALG_COMPACT 1
-#endif
 constexpr int kTileWarps = 8;              // warps per CTA of every kernel using warp-blocks
 constexpr int kTileSmemDoubles = 13 * 32;  // per warp: column state [7][32], sums [6][32]
 
@@ -328,9 +310,6 @@ __device__ __forceinline__ void warp_block_solve_compact(const double *x, const 
 // CTA must call it (warps without a block pass live = false); ws is the warp's slice of
 // phase_slice_doubles<kBalanced>() doubles: column states [7][32], column sums [6][32], and
 // for the balanced loops row states [7][32] and row sums [6][32].
-#ifndef BIA_PHASE_WARPS
-#define BIA_PHASE_WARPS 32  // 0: never use the phase-locked kernels
-#endif
 constexpr int kPhaseSliceDoubles = kTileSmemDoubles + 13 * 32;
 // a phase-locked warp's slice: the balanced loops add the rows to the column slice; the
 // per-lane loops keep the rows in registers and leave the rest of the SM's on-chip memory to
@@ -697,46 +676,8 @@ __device__ __forceinline__ void warp_block_solve(const double *x, const double *
                                                  int bi, int bj, int lane, double racc[6], double cacc[6],
                                                  PairCounters &cnt)
 {
-    if (M == kMethodAlg && BIA_ALG_COMPACT) {
-        warp_block_solve_compact(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
-        return;
-    }
-    if (M == kMethodRkf && BIA_RKF_SMEM) {
-        warp_block_solve_rkf(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
-        return;
-    }
-    const unsigned full = 0xffffffffu;
-    const int i = bi * 32 + lane;
-    double si[7], sj[7];
-    load_particle(x, y, z, u, v, w, q, n, i, si);
-    load_particle(x, y, z, u, v, w, q, n, bj * 32 + lane, sj);
-#pragma unroll
-    for (int c = 0; c < 6; c++) racc[c] = cacc[c] = 0.0;
-    counters_zero(cnt);
-    const bool diag = (bi == bj);
-    const int k0 = diag ? 1 : 0;
-    const int k1 = diag ? 16 : 31;
-    for (int k = k0; k <= k1; k++) {
-        const int src = (lane + k) & 31;
-        double sc[7];
-#pragma unroll
-        for (int c = 0; c < 7; c++) sc[c] = __shfl_sync(full, sj[c], src);
-        const int j = bj * 32 + src;
-        const bool active = (!diag || k < 16 || lane < 16) && i < n && j < n;
-        double h[6] = {0, 0, 0, 0, 0, 0};
-        if (active) {
-            const double r[3] = {si[0] - sc[0], si[1] - sc[1], si[2] - sc[2]};
-            const double g[3] = {si[3] - sc[3], si[4] - sc[4], si[5] - sc[5]};
-            const double eps_ij = q ? eps_th * si[6] * sc[6] : eps_th;
-            pair_halfdisp<M>(P, eps_ij, r, g, h, cnt);
-        }
-        const int back = (lane - k) & 31;
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-            racc[c] += h[c];
-            cacc[c] += __shfl_sync(full, h[c], back);
-        }
-    }
+    if (M == kMethodAlg) warp_block_solve_compact(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
+    else warp_block_solve_rkf(x, y, z, u, v, w, q, n, eps_th, P, bi, bj, lane, racc, cacc, cnt);
 }
 
 // Deterministic partial layout part[m][c][p] (plane = padded particle count): row sums
