@@ -57,18 +57,19 @@ if ROOT not in sys.path:
 # Algorithmic FP64 flops per pair (convention: + - * / sqrt = 1, FMA = 2, each libm
 # transcendental = 20, sincos = 40), counted from the reference's formulas:
 # base cost per pair of each branch (frame + classification + solve set-up + finish +
-# half-displacement + accumulation) and the cost of one solver iteration.
+# half-displacement + accumulation) and the cost of one solver iteration.  The kernels' own
+# forms of the conic and RKF45 branches take fewer operations than these.
 FLOPS = {
     "hyperbola": (661, 125),   # per pair, per main-loop Newton iteration
     "ellipse": (447, 47),      # per pair, per Kepler Newton step
     "parabola": (429, 76),     # per pair, per Barker Newton step
     "rkf": (147, 758),         # per pair, per accepted RKF45 step (3 Fehlberg stages sets)
-    # universal variables (this library's solver, not the reference's), counted from the
-    # dimensionless series form every exact pair takes: differences 6, prepare 20 (|r|^2,
-    # r.g, |g|^2, rsqrt as sqrt + division, beta), series with its exactness test 41,
-    # composition with the three-term Stumpff series and the series of r0/r 63, accumulation
-    # 12 per pair; 43 per Newton iteration (almost none at the benchmark steps)
-    "universal": (142, 43),
+    # universal variables (this library's solver, not the reference's), FP64 operations of the
+    # short-step pair that nearly every pair of these workloads is: differences 6, |r|^2, r.w,
+    # |w|^2, 1/r, U, a, q 23, the four series' FP64 terms 24, the factors and the six
+    # displacements 22, accumulation 12 (and about 45 in FP32); 43 per Newton iteration of the
+    # others (their prepare, series and composition, 142, are counted as a short-step pair's)
+    "universal": (87, 43),
     "learned": (330, 0),       # per learned pair: elements, FP64 Halley step, composition
 }
 # BF16 tensor-core flops per learned pair: 2 x (16 x 64 + 64 x 64 + 64 x 64) multiply-adds
@@ -79,7 +80,7 @@ METHODS = {"rkf": 0, "alg": 1, "universal": 2, "learned": 3}
 # kernel, from one ncu capture at n = 16384 of the same workload and method, scaled by the
 # pairs per launch (both the partial sums and any local-memory traffic grow with the pairs):
 #   (workload, method, learned layout) -> (pairs in the capture, bytes in the capture)
-# The learned step's dominant kernel is the rest kernel (it writes every partial slot; the head
+# The learned step's dominant kernel is the rest pass's walk (it writes every partial slot; the head
 # and finish kernels move under 1 MB at this size on this workload).
 TRAFFIC = {
     ("plummer_32768", 3, "split"): (16384 * 16383 // 2, 1.049e6 + 345.274e6),
@@ -659,17 +660,18 @@ def main():
     else:  # the library's rule: the learned step splits at every size
         split = method == 3
     if method == 3:
-        kernel_name = ("bia_pair_rest_kernel<true> + bia_pair_learned_head_kernel + "
+        kernel_name = ("bia_pair_walk_kernel<true, true> + bia_pair_learned_head_kernel + "
                        "bia_pair_learned_finish_kernel<true> (one timed interval)"
                        if split else "bia_pair_learned_kernel<true>")
-    elif method == 1 and tuned is not None:
-        kernel_name = {"tiles8": "bia_pair_tiles_kernel<true, 1>",
+    elif method == 1:
+        per_sm = nwb / sms
+        shape = (tuned["alg_shape"] if tuned is not None
+                 else "phase32" if 24 <= per_sm <= 32 or per_sm >= 48 else "tiles8")
+        kernel_name = {"tiles8": "bia_pair_block_kernel<true>" if per_sm < 48 else "bia_pair_tiles_kernel<true>",
                        "phase32_lane": "bia_pair_phase_kernel<true, 32, 1, false>",
-                       "phase32": "bia_pair_phase_kernel<true, 32, 1, true>"}[tuned["alg_shape"]]
-    elif method == 1 and (nwb + 31) // 32 >= 2 * sms:
-        kernel_name = "bia_pair_phase_kernel<true, 32, 1>"
+                       "phase32": "bia_pair_phase_kernel<true, 32, 1, true>"}[shape]
     else:
-        kernel_name = "bia_pair_tiles_kernel<true, %d>" % method
+        kernel_name = "bia_pair_block_rkf_kernel<true>" if method == 0 else "bia_pair_walk_kernel<true, false>"
     flops_total = pair_flops(stats, method)
     per_launch_flops = flops_total / max(kern_launches, 1)
     per_launch_s = kern_ms * 1e-3 / max(kern_launches, 1)

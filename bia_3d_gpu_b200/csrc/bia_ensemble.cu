@@ -412,7 +412,8 @@ __global__ void __launch_bounds__(256) ens_energy_kernel(const double *u, const 
 //                SM) with per-lane class loops, 2: the same with the balanced class loops;
 //                built-in rule: 2 from two of its CTAs per SM up, else 0
 //   universal    0: one item per warp, 1: a persistent grid of 2 CTAs per SM (built-in)
-//   learned      the persistent head kernel with 0: 1 CTA per SM, 1: 2 CTAs per SM (built-in)
+//   learned      the persistent head kernel with 0: 1 CTA per SM, 1: all that are resident
+//                (built-in; four per SM, two when the shape got its name)
 // Every shape runs the same per-item arithmetic in the same order: the results are bitwise
 // the same.
 constexpr int kEnsShapes = 3;
@@ -442,7 +443,7 @@ static int ens_pair_launch(bia_context *ctx, bia_ensemble *E, EnsArgs &A, int me
         const unsigned rgrid = (unsigned)persistent_grid(grid);
         ens_pair_walk_kernel<true><<<rgrid, kEnsThreads, walk_smem_bytes<true>(kEnsWarps), st>>>(A);
         long long hcap = lsetup;
-        if (shape == 0 || shape == 1) hcap = (long long)device_sm_count() * (shape + 1);
+        if (shape == 0) hcap = device_sm_count();
         launch_learned_head(A.R, A.heads, A.stats, (int)hcap, st);
         ens_pair_learned_finish_kernel<<<rgrid, kEnsThreads, 0, st>>>(A);
         return cuda_status(cudaGetLastError());

@@ -347,7 +347,7 @@ static int alg_variant_for(long long nwb, int tuned)
     return one_wave || nwb >= kBlockMaxPerSm * sms ? kVarPhase32 : kVarTiles8;
 }
 
-// CTAs per SM of the persistent universal-variable and rest kernels (their launch bound)
+// CTAs per SM of the persistent walk kernels (their launch bound)
 constexpr int kPersistentCtas = 2;
 
 // SM count of the current device (cached per device); 0 when the query fails
