@@ -672,6 +672,8 @@ def main():
                        "phase32": "bia_pair_phase_kernel<true, 32, 1, true>"}[shape]
     else:
         kernel_name = "bia_pair_block_rkf_kernel<true>" if method == 0 else "bia_pair_walk_kernel<true, false>"
+    if nwb <= 2 * sms:
+        kernel_name = kernel_name.replace("pair_walk_kernel", "pair_walk_block_kernel")
     flops_total = pair_flops(stats, method)
     per_launch_flops = flops_total / max(kern_launches, 1)
     per_launch_s = kern_ms * 1e-3 / max(kern_launches, 1)

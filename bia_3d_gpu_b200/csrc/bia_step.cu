@@ -298,6 +298,9 @@ constexpr int phase_smem_bytes()
     return kW * (phase_slice_doubles<kBalanced>() + kNumStats) * (int)sizeof(double);
 }
 
+template <bool kDeterministic, bool kRest>
+__global__ void bia_pair_walk_block_kernel(const StepArgs A);
+
 // Once per device (the current one): opt the phase-locked kernels in to their dynamic
 // shared memory and read the SM count.  Returns the SM count, 0 when the set-up failed
 // (the caller then launches the 8-warp kernel).
@@ -329,6 +332,14 @@ static int phase_kernel_setup()
                                         (int)sizeof(RkfBlockShared)) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(bia_pair_block_rkf_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sizeof(RkfBlockShared)) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)walk_block_smem_bytes<false>()) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)walk_block_smem_bytes<false>()) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)walk_block_smem_bytes<true>()) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)walk_block_smem_bytes<true>()) == cudaSuccess;
         if (!ok) cudaGetLastError();  // clear; the 8-warp kernel is used instead
         sms_of[dev] = ok ? sms : 0;
         done_of[dev] = true;
@@ -419,6 +430,34 @@ __global__ void __launch_bounds__(kThreads, kPersistentCtas) bia_pair_walk_kerne
     walk_flush_counts(c, A.stats, lane);
 }
 
+// The same by a CTA per warp-block (uv_block_solve), up to kWalkBlockMaxPerSm warp-blocks per SM, one wave of
+// resident CTAs: a second wave costs more than the walk's longer chain where many pairs are left to
+// a CTA's one warp.  Measured, us a graph-replayed step, walk | block: Plummer, universal, n = 2, 33, 257, 500: 9.3 |
+// 6.5, 13.7 | 8.4, 17.4 | 10.6, 18.6 | 11.1, of 750 (300 warp-blocks) 19.4 | 14.6, of 1332 21.5 | 28.5; at a step
+// of 1e-2 (every pair left) of 500 51 | 42, of 750 58 | 70; learned, 257: 43.9 | 38.2, of 1332 55 | 64.
+constexpr long long kWalkBlockMaxPerSm = 2;
+
+template <bool kDeterministic, bool kRest>
+__global__ void __launch_bounds__(kWalkBlockWarps * 32, 2) bia_pair_walk_block_kernel(const StepArgs A)
+{
+    WalkCounts c = {0, 0, 0, 0};
+    uv_block_solve<kDeterministic, kRest>(StepItems{A}, blockIdx.x, A.P.dt, A.R, c);
+    if (threadIdx.x < 32) walk_flush_counts(c, A.stats, threadIdx.x);
+}
+
+template <bool kDeterministic, bool kRest>
+static void launch_pair_walk(const StepArgs &A, cudaStream_t st)
+{
+    if (A.nwb <= kWalkBlockMaxPerSm * phase_kernel_setup()) {
+        bia_pair_walk_block_kernel<kDeterministic, kRest>
+            <<<(unsigned)A.nwb, kWalkBlockWarps * 32, walk_block_smem_bytes<kRest>(), st>>>(A);
+        return;
+    }
+    const long long grid = persistent_grid((A.nwb + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    bia_pair_walk_kernel<kDeterministic, kRest>
+        <<<(unsigned)grid, kThreads, walk_smem_bytes<kRest>(kWarpsPerBlock), st>>>(A);
+}
+
 template <bool kDeterministic>
 static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st, int tuned = -1)
 {
@@ -447,8 +486,7 @@ static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st
             <<<(unsigned)(A.nwb < 0x7fffffffLL ? A.nwb : 0x7fffffffLL), kBlockWarps * 32, sizeof(RkfBlockShared), st>>>(A);
         break;
     case kMethodUniversal:
-        bia_pair_walk_kernel<kDeterministic, false>
-            <<<(unsigned)persistent_grid(grid), kThreads, walk_smem_bytes<false>(kWarpsPerBlock), st>>>(A);
+        launch_pair_walk<kDeterministic, false>(A, st);
         break;
     default:
         bia_pair_tiles_kernel<kDeterministic><<<(unsigned)grid, kThreads, 0, st>>>(A);
@@ -689,9 +727,7 @@ static int launch_pair_learned(const StepArgs &A, cudaStream_t st)
     }
     // the row counts of both heads and the list length start at zero
     if (cudaMemsetAsync(A.R.counts, 0, kSplitHeader, st) != cudaSuccess) return BIA_ERR_CUDA;
-    const long long rgrid = persistent_grid((A.nwb + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    bia_pair_walk_kernel<kDeterministic, true>
-        <<<(unsigned)rgrid, kThreads, walk_smem_bytes<true>(kWarpsPerBlock), st>>>(A);
+    launch_pair_walk<kDeterministic, true>(A, st);
     launch_learned_head(A.R, A.heads, A.stats, lgrid, st);
     const long long fgrid = persistent_grid((A.nwb + kWarpsPerBlock - 1) / kWarpsPerBlock);
     bia_pair_learned_finish_kernel<kDeterministic><<<(unsigned)fgrid, kThreads, 0, st>>>(A);

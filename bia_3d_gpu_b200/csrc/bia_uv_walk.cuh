@@ -344,6 +344,195 @@ __device__ __forceinline__ void walk_queue(const Items &I, const LearnedRows &R,
     __syncwarp();
 }
 
+// What a block's sums lack after its first pass: the half-displacement's constant factors, and
+// velocities over dt (uv_fast_pair).
+__device__ __forceinline__ void walk_scale(const UvFastStep &T, double *ws, int lane, double racc[6])
+{
+    const double sv = 0.5 / T.dt;
+    double2 *acc = slice_sums(ws);
+    double2 a = acc[lane];
+    acc[lane] = make_double2(0.25 * a.x, 0.25 * a.y);
+    a = acc[32 + lane];
+    acc[32 + lane] = make_double2(0.25 * a.x, sv * a.y);
+    a = acc[64 + lane];
+    acc[64 + lane] = make_double2(sv * a.x, sv * a.y);
+#pragma unroll
+    for (int d = 0; d < 6; d++) racc[d] *= d < 3 ? 0.25 : sv;
+    __syncwarp();
+}
+
+// A block after its first pass (sums racc and the slice's, the pairs in `left` unsolved): many others, or a
+// diagonal block, finished on the spot; its sums written.  Returns how many are left for the queue.
+template <bool kDeterministic, bool kRest>
+__device__ __forceinline__ unsigned walk_block_finish(const WalkSystem &S, const WalkBlock &B, unsigned left, double racc[6],
+                                                      double *ws, uint32_t *wslots, const LearnedRows &R, double dt,
+                                                      int lane, WalkCounts &c)
+{
+    const bool diag = B.bi == B.bj;
+    const int i = B.bi * 32 + lane, j = B.bj * 32 + lane;
+    c.pairs += block_lane_pairs(lane, B.bi, B.bj, S.n);
+    unsigned others = __reduce_add_sync(0xffffffffu, (unsigned)__popc(left));
+    if (others != 0u && (diag || others > (unsigned)kQueuePairs)) {  // finished on the spot
+        double si[7], sj[7];
+        load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, i, si);
+        load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, j, sj);
+        slice_states(ws, lane, sj);
+        __syncwarp();
+        uint32_t mask[kMlpHeads] = {0u, 0u};
+        auto other = [&](int src, int k, const double *row, double *h) {
+            double r[3], g[3];
+            const double eps_ij = slice_pair(ws, src, row, S.q != nullptr, S.eps_th, r, g);
+            uint32_t x01 = 0u;
+            const int kind = walk_other_pair<kRest>(eps_ij, dt, r, g, h, x01, c);
+            if (kRest && kind != kLearnedPlain) {
+                mask[kHeadHyp] |= (kind == kLearnedHyp ? 1u : 0u) << k;
+                mask[kHeadEll] |= (kind == kLearnedHyp ? 0u : 1u) << k;
+                wslots[lane * 32 + k] = x01;
+            }
+        };
+        uv_walk_rest(left, ws, lane, si, racc, other);
+        if (kRest) rest_block_defer(R, B.item, mask, wslots, lane);
+        others = 0u;
+    }
+    double cacc[6];
+    slice_sums_of(ws, lane, cacc);
+    walk_write<kDeterministic>(S, B.bi, B.bj, lane, racc, cacc);
+    __syncwarp();  // the slice is reused by the next block; the sums are there for the queue
+    return others;
+}
+
+// the pairs in `left` of block B, the queue's nblocks-th, behind the qn pairs there
+__device__ __forceinline__ void walk_queue_push(unsigned int *queue, WalkBlock *blocks, const WalkBlock &B, unsigned left,
+                                                int qn, int nblocks, int lane)
+{
+    unsigned incl = (unsigned)__popc(left);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
+    }
+    int at = qn + (int)incl - __popc(left);
+    for (unsigned m = left; m; m &= m - 1u)
+        queue[at++] = ((unsigned)nblocks << 10) | ((unsigned)(__ffs(m) - 1) << 5) | (unsigned)lane;
+    if (lane == 0) blocks[nblocks] = B;
+    __syncwarp();
+}
+
+// lane's pairs of a block, bit k (no short step)
+__device__ __forceinline__ unsigned walk_all_pairs(bool diag, int lane, bool row_live, int ncols)
+{
+    unsigned left = 0u;
+    const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
+    for (int k = k0; k <= k1; k++)
+        if ((!diag || k < 16 || lane < 16) && row_live && ((lane + k) & 31) < ncols) left |= 1u << k;
+    return left;
+}
+
+// One block by a CTA of kWalkBlockWarps warps (small systems, where a warp's 32 offsets in a row are most of
+// a step): the warps solve the first pass's pairs of four offsets each, every h waits in shared memory, and a
+// warp per component adds the rows and the columns in offset order; warp 0 does the rest of the
+// block as the walk does.  The same sums, bitwise.  Dynamic shared memory, in doubles: warp 0's slice and
+// queue as the walk's, the row sums, the masks of pairs left, the h.
+constexpr int kWalkBlockWarps = 8;
+template <bool kRest>
+__host__ __device__ constexpr size_t walk_block_smem_bytes()
+{
+    return (size_t)(walk_warp_doubles<kRest>() + 6 * 32 + 16 + 6 * 1024) * sizeof(double);
+}
+
+template <bool kDeterministic, bool kRest, class Items>
+__device__ __forceinline__ void uv_block_solve(const Items &I, long long t, double dt, const LearnedRows &R, WalkCounts &c)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *ws = warp_slices;
+    WalkBlock *blocks = reinterpret_cast<WalkBlock *>(ws + kTileSmemDoubles);
+    unsigned int *queue = reinterpret_cast<unsigned int *>(blocks + kQueuePairs);
+    uint32_t *wslots = reinterpret_cast<uint32_t *>(ws + kWalkSliceDoubles);
+    double *rsums = ws + walk_warp_doubles<kRest>();
+    unsigned *lefts = reinterpret_cast<unsigned *>(rsums + 6 * 32);
+    double *hs = rsums + 6 * 32 + 16;
+    const UvFastStep T = uv_fast_step(dt);
+    const WalkBlock B = I.block(t);
+    const WalkSystem S = I.system(B.sys);
+    const bool diag = B.bi == B.bj;
+    const int i = B.bi * 32 + lane, ncols = S.n - B.bj * 32;
+    const bool full_block = !diag && ncols >= 32;
+    const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
+    UvRow row;
+    {
+        double si[7];
+        load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, i, si);
+        row.cdt2 = S.q ? S.eps_th * T.dt2 * si[6] : S.eps_th * T.dt2;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            row.s[d] = si[d];
+            row.s[3 + d] = si[3 + d] * T.dt;
+        }
+    }
+    if (warp == 0) {
+        double sj[7];
+        load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, B.bj * 32 + lane, sj);
+#pragma unroll
+        for (int d = 3; d < 6; d++) sj[d] *= T.dt;
+        slice_fill(ws, lane, sj);
+        lefts[lane] = 0u;
+    }
+    __syncthreads();
+    if (T.on) {  // the same for the CTA
+        unsigned mine = 0u;
+        for (int k = k0 + warp; k <= k1; k += kWalkBlockWarps) {
+            const int src = (lane + k) & 31;
+            const bool active = full_block || ((!diag || k < 16 || lane < 16) && i < S.n && src < ncols);
+            double r[3], w[3], h[6];
+            slice_diff(ws, src, row.s, r, w);
+            const bool ok = uv_fast_pair(S.q ? row.cdt2 * ws[6 * 32 + src] : row.cdt2, r, w, h);
+            mine |= (active && !ok ? 1u : 0u) << k;
+#pragma unroll
+            for (int d = 0; d < 6; d++) hs[1024 * d + 32 * k + lane] = active && ok ? h[d] : 0.0;
+        }
+        if (mine) atomicOr(&lefts[lane], mine);
+        __syncthreads();
+        if (warp < 6) {
+            unsigned left = lefts[lane];
+            int last = k1;  // the walk stops after kProbe offsets of a long step's block
+            if (full_block && __reduce_add_sync(0xffffffffu, (unsigned)__popc(left & ((1u << kProbe) - 1u))) > 32u * kProbe / 4u)
+                last = kProbe - 1;
+            const double *h = hs + 1024 * warp;
+            double rsum = 0.0, csum = 0.0;
+#pragma unroll 8
+            for (int k = k0; k <= last; k++) {
+                rsum += h[32 * k + lane];
+                csum += h[32 * k + ((lane - k) & 31)];
+            }
+            rsums[32 * warp + lane] = rsum;
+            double2 *acc = slice_sums(ws) + (warp >> 1) * 32 + lane;
+            if (warp & 1) acc->y = csum;
+            else acc->x = csum;
+        }
+        __syncthreads();
+    }
+    if (warp != 0) return;
+    unsigned left;
+    double racc[6];
+    if (T.on) {
+        left = lefts[lane];
+        if (full_block && __reduce_add_sync(0xffffffffu, (unsigned)__popc(left & ((1u << kProbe) - 1u))) > 32u * kProbe / 4u)
+            left |= 0xffffffffu << kProbe;
+#pragma unroll
+        for (int d = 0; d < 6; d++) racc[d] = rsums[32 * d + lane];
+        walk_scale(T, ws, lane, racc);
+    } else {
+#pragma unroll
+        for (int d = 0; d < 6; d++) racc[d] = 0.0;
+        left = walk_all_pairs(diag, lane, i < S.n, ncols);
+    }
+    const unsigned others = walk_block_finish<kDeterministic, kRest>(S, B, left, racc, ws, wslots, R, dt, lane, c);
+    if (others != 0u) {
+        walk_queue_push(queue, blocks, B, left, 0, 0, lane);
+        walk_queue<kDeterministic, kRest>(I, R, dt, queue, blocks, (int)others, lane, c);
+    }
+}
+
 // The walk of a persistent grid: warp `first` of `stride` warps takes blocks first, first + stride, ... of
 // `count`.  I.block(t) gives block t, I.system(s) a system; `slice` is where the warp's doubles
 // (walk_warp_doubles) begin in the dynamic shared memory.
@@ -351,7 +540,6 @@ template <bool kDeterministic, bool kRest, class Items>
 __device__ __forceinline__ void uv_walk_blocks(const Items &I, long long first, long long stride, long long count,
                                                double dt, int slice, const LearnedRows &R, WalkCounts &c)
 {
-    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     double *ws = warp_slices + slice;
     WalkBlock *blocks = reinterpret_cast<WalkBlock *>(ws + kTileSmemDoubles);
@@ -391,52 +579,12 @@ __device__ __forceinline__ void uv_walk_blocks(const Items &I, long long first, 
                         left = S.q ? uv_walk_part<true>(slice, row, lane, diag, i < S.n, ncols, racc)
                                    : uv_walk_part<false>(slice, row, lane, diag, i < S.n, ncols, racc);
                     }
-                    // the half-displacement's constant factors, and velocities over dt (uv_fast_pair)
-                    const double sv = 0.5 / T.dt;
-                    double2 *acc = slice_sums(ws);
-                    double2 a = acc[lane];
-                    acc[lane] = make_double2(0.25 * a.x, 0.25 * a.y);
-                    a = acc[32 + lane];
-                    acc[32 + lane] = make_double2(0.25 * a.x, sv * a.y);
-                    a = acc[64 + lane];
-                    acc[64 + lane] = make_double2(sv * a.x, sv * a.y);
-#pragma unroll
-                    for (int d = 0; d < 6; d++) racc[d] *= d < 3 ? 0.25 : sv;
-                    __syncwarp();
+                    walk_scale(T, ws, lane, racc);
                 } else {
-                    const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
-                    for (int k = k0; k <= k1; k++)
-                        if ((!diag || k < 16 || lane < 16) && i < S.n && ((lane + k) & 31) < ncols) left |= 1u << k;
+                    left = walk_all_pairs(diag, lane, i < S.n, ncols);
                 }
             }
-            c.pairs += block_lane_pairs(lane, B.bi, B.bj, S.n);
-            others = __reduce_add_sync(full, (unsigned)__popc(left));
-            if (others != 0u && (diag || others > (unsigned)kQueuePairs)) {  // finished on the spot
-                double si[7], sj[7];
-                load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, i, si);
-                load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, j, sj);
-                slice_states(ws, lane, sj);
-                __syncwarp();
-                uint32_t mask[kMlpHeads] = {0u, 0u};
-                auto other = [&](int src, int k, const double *row, double *h) {
-                    double r[3], g[3];
-                    const double eps_ij = slice_pair(ws, src, row, S.q != nullptr, S.eps_th, r, g);
-                    uint32_t x01 = 0u;
-                    const int kind = walk_other_pair<kRest>(eps_ij, dt, r, g, h, x01, c);
-                    if (kRest && kind != kLearnedPlain) {
-                        mask[kHeadHyp] |= (kind == kLearnedHyp ? 1u : 0u) << k;
-                        mask[kHeadEll] |= (kind == kLearnedHyp ? 0u : 1u) << k;
-                        wslots[lane * 32 + k] = x01;
-                    }
-                };
-                uv_walk_rest(left, ws, lane, si, racc, other);
-                if (kRest) rest_block_defer(R, B.item, mask, wslots, lane);
-                others = 0u;
-            }
-            double cacc[6];
-            slice_sums_of(ws, lane, cacc);
-            walk_write<kDeterministic>(S, B.bi, B.bj, lane, racc, cacc);
-            __syncwarp();  // the slice is reused by the next block; the sums are there for the queue
+            others = walk_block_finish<kDeterministic, kRest>(S, B, left, racc, ws, wslots, R, dt, lane, c);
         }
         if (qn != 0 && (!have || qn + (int)others > kQueuePairs)) {
             walk_queue<kDeterministic, kRest>(I, R, dt, queue, blocks, qn, lane, c);
@@ -444,19 +592,9 @@ __device__ __forceinline__ void uv_walk_blocks(const Items &I, long long first, 
         }
         if (!have) return;
         if (others != 0u) {
-            unsigned incl = (unsigned)__popc(left);
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const unsigned o = __shfl_up_sync(full, incl, d);
-                if (lane >= d) incl += o;
-            }
-            int at = qn + (int)incl - __popc(left);
-            for (unsigned m = left; m; m &= m - 1u)
-                queue[at++] = ((unsigned)nblocks << 10) | ((unsigned)(__ffs(m) - 1) << 5) | (unsigned)lane;
-            if (lane == 0) blocks[nblocks] = B;
+            walk_queue_push(queue, blocks, B, left, qn, nblocks, lane);
             nblocks++;
             qn += (int)others;
-            __syncwarp();
         }
     }
 }
