@@ -14,6 +14,7 @@
 // over all I, from Python), now 45.
 #include <cuda_runtime.h>
 
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 
@@ -77,46 +78,44 @@ __global__ void __launch_bounds__(32) bia_row_kernel(const RowArgs A)
     if (lane == 0) part[6] = nonfinite;
 }
 
-// A host thread's pinned buffer, grown on demand.  A thread that ends leaves it, linked through
-// the buffer's own first bytes, to the next one that starts: at most as many are held as threads
-// have used the entry at the same time.  They die with the process; freeing them here could run
-// after the CUDA runtime has shut down.
-struct IdleBuffer {
-    IdleBuffer *next;
+// A host thread's pinned buffer, grown on demand.  A thread that ends leaves it to the next one that
+// starts: at most as many are held as threads have used the entry at the same time.  They die with
+// the process; freeing them here could run after the CUDA runtime has shut down.  What is known of a
+// buffer lies beside it, so that a buffer that died early (a device reset) is never read here.
+struct RowBuffer {
+    RowBuffer *next;
+    double *ptr;
     size_t bytes;
 };
 static std::mutex g_idle_lock;
-static IdleBuffer *g_idle = nullptr;
+static RowBuffer *g_idle = nullptr;
 
 struct RowState {
-    double *ptr = nullptr;
-    size_t bytes = 0;
+    RowBuffer *buf = nullptr;
     ~RowState()
     {
-        if (!ptr) return;
+        if (!buf) return;
         std::lock_guard<std::mutex> g(g_idle_lock);
-        IdleBuffer *b = (IdleBuffer *)ptr;
-        b->next = g_idle;
-        b->bytes = bytes;
-        g_idle = b;
+        buf->next = g_idle;
+        g_idle = buf;
     }
     cudaError_t reserve(size_t want)
     {
-        if (want <= bytes) return cudaSuccess;
-        if (!ptr) {
+        if (!buf) {
             std::lock_guard<std::mutex> g(g_idle_lock);
             if (g_idle) {
-                ptr = (double *)g_idle;
-                bytes = g_idle->bytes;
-                g_idle = g_idle->next;
+                buf = g_idle;
+                g_idle = buf->next;
             }
         }
-        if (want <= bytes) return cudaSuccess;
-        if (ptr) cudaFreeHost(ptr);
-        ptr = nullptr;
-        bytes = 0;
-        cudaError_t e = cudaHostAlloc((void **)&ptr, want, cudaHostAllocMapped | cudaHostAllocPortable);
-        if (e == cudaSuccess) bytes = want;
+        if (!buf) buf = (RowBuffer *)calloc(1, sizeof(RowBuffer));
+        if (!buf) return cudaErrorMemoryAllocation;
+        if (want <= buf->bytes) return cudaSuccess;
+        if (buf->ptr && cudaFreeHost(buf->ptr) != cudaSuccess) cudaGetLastError();  // clear
+        buf->ptr = nullptr;
+        buf->bytes = 0;
+        cudaError_t e = cudaHostAlloc((void **)&buf->ptr, want, cudaHostAllocMapped | cudaHostAllocPortable);
+        if (e == cudaSuccess) buf->bytes = want;
         return e;
     }
 };
@@ -145,14 +144,15 @@ extern "C" void find_dxyuv_kernel_(const int METHOD, const int N, const int I, c
     const size_t span = ((size_t)6 * N + 31) / 32 * 32;
     cudaError_t e = S.reserve((2 * span + (size_t)kRowPart * ((N + 31) / 32)) * sizeof(double));
     double *d_buf = nullptr;
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&d_buf, S.ptr, 0);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&d_buf, S.buf->ptr, 0);
     if (e != cudaSuccess) {
         set_last_error(cuda_status(e));
         return;
     }
-    const double *out = S.ptr + span, *part = S.ptr + 2 * span;
+    double *const rel = S.buf->ptr;
+    const double *out = rel + span, *part = rel + 2 * span;
     if (m > 0) {
-        memcpy(S.ptr, RXYZUVW + below, words * sizeof(double));
+        memcpy(rel, RXYZUVW + below, words * sizeof(double));
         RowArgs A;
         A.rel = d_buf;
         A.out = d_buf + span;

@@ -1382,7 +1382,7 @@ int bia_run(bia_context *ctx, const bia_config *cfg, int n, double *x, double *y
     if (use_graph && ctx->stream && !ctx->timing && nsteps > 0) {
         // one-time kernel attribute set-up happens before the capture begins
         if (cfg->method == BIA_METHOD_LEARNED && !learned_kernel_setup()) return BIA_ERR_CUDA;
-        if (cfg->method == BIA_METHOD_ALG) phase_kernel_setup();
+        phase_kernel_setup();
         GraphKey key;
         key.n = n; key.nsteps = nsteps; key.method = cfg->method; key.itr = cfg->itr;
         key.deterministic = cfg->deterministic; key.eps = cfg->eps_th; key.dt = cfg->dt;
