@@ -1132,7 +1132,9 @@ static int dim_integrate_coop(DimRun &R, double *y, double *x0, double xe, int i
     const int cap = gcap ? atoi(gcap) : 0;
     if (cap <= 0 && dim_resident_plan(R.n, sms, (size_t)max_smem, B, &G, &reg, &bytes)) {
         kern = R.fast_inv ? dim_resident_form<true>(reg) : dim_resident_form<false>(reg);
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+        // the limit belongs to the process: always the device's own, so that no call takes room from one that
+        // another thread is about to launch
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
