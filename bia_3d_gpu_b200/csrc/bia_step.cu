@@ -24,6 +24,7 @@
 // partials are [nb][6][nb*32] FP64 (1.5 n^2 bytes); accumulators [6][nb*32].
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -301,48 +302,50 @@ constexpr int phase_smem_bytes()
 template <bool kDeterministic, bool kRest>
 __global__ void bia_pair_walk_block_kernel(const StepArgs A);
 
-// Once per device (the current one): opt the phase-locked kernels in to their dynamic
-// shared memory and read the SM count.  Returns the SM count, 0 when the set-up failed
-// (the caller then launches the 8-warp kernel).
-static int phase_kernel_setup()
+// A kernel's opt-in to `bytes` of dynamic shared memory on the current device.
+template <class Kernel>
+static bool smem_opt_in(Kernel *kernel, size_t bytes)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
+
+// Contexts created so far: a device reset forgets the opt-ins, and what runs after one runs on
+// contexts created after it.
+static std::atomic<unsigned> g_contexts{0};
+
+// Once per device (the current one) and again after a context was created: opt the pair kernels in to their
+// dynamic shared memory and read the SM count.  Returns the SM count, 0 when the set-up failed
+// (the caller then launches the 8-warp kernel).  if_made: only where the set-up was made
+// before (a new context makes it again; the first one leaves it, and the kernels' loading, to the first step).
+static int phase_kernel_setup(bool if_made = false)
 {
     constexpr int kMaxDevices = 64;
     static std::mutex mu;
     static int sms_of[kMaxDevices] = {};
-    static bool done_of[kMaxDevices] = {};
+    static unsigned made_of[kMaxDevices] = {};  // 1 + g_contexts at the set-up
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     std::lock_guard<std::mutex> lk(mu);
-    if (!done_of[dev]) {
+    const unsigned now = 1u + g_contexts.load();
+    if (if_made && made_of[dev] == 0u) return 0;
+    if (made_of[dev] != now) {
         int sms = 0;
-        bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_phase_kernel<true, 32, 1>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, phase_smem_bytes<32>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_phase_kernel<false, 32, 1>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, phase_smem_bytes<32>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_phase_kernel<true, 32, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        phase_smem_bytes<32, false>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_phase_kernel<false, 32, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        phase_smem_bytes<32, false>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(AlgBlockShared)) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_block_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(AlgBlockShared)) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_block_rkf_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(RkfBlockShared)) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_block_rkf_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(RkfBlockShared)) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)walk_block_smem_bytes<false>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)walk_block_smem_bytes<false>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)walk_block_smem_bytes<true>()) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(bia_pair_walk_block_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)walk_block_smem_bytes<true>()) == cudaSuccess;
+        const bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+                        smem_opt_in(bia_pair_phase_kernel<true, 32, 1>, phase_smem_bytes<32>()) &&
+                        smem_opt_in(bia_pair_phase_kernel<false, 32, 1>, phase_smem_bytes<32>()) &&
+                        smem_opt_in(bia_pair_phase_kernel<true, 32, 1, false>, phase_smem_bytes<32, false>()) &&
+                        smem_opt_in(bia_pair_phase_kernel<false, 32, 1, false>, phase_smem_bytes<32, false>()) &&
+                        smem_opt_in(bia_pair_block_kernel<true>, sizeof(AlgBlockShared)) &&
+                        smem_opt_in(bia_pair_block_kernel<false>, sizeof(AlgBlockShared)) &&
+                        smem_opt_in(bia_pair_block_rkf_kernel<true>, sizeof(RkfBlockShared)) &&
+                        smem_opt_in(bia_pair_block_rkf_kernel<false>, sizeof(RkfBlockShared)) &&
+                        smem_opt_in(bia_pair_walk_block_kernel<true, false>, walk_block_smem_bytes<false>()) &&
+                        smem_opt_in(bia_pair_walk_block_kernel<false, false>, walk_block_smem_bytes<false>()) &&
+                        smem_opt_in(bia_pair_walk_block_kernel<true, true>, walk_block_smem_bytes<true>()) &&
+                        smem_opt_in(bia_pair_walk_block_kernel<false, true>, walk_block_smem_bytes<true>());
         if (!ok) cudaGetLastError();  // clear; the 8-warp kernel is used instead
         sms_of[dev] = ok ? sms : 0;
-        done_of[dev] = true;
+        made_of[dev] = now;
     }
     return sms_of[dev];
 }
@@ -445,10 +448,12 @@ __global__ void __launch_bounds__(kWalkBlockWarps * 32, 2) bia_pair_walk_block_k
     if (threadIdx.x < 32) walk_flush_counts(c, A.stats, threadIdx.x);
 }
 
+// renew, here and below: the launched kernel's opt-in is made again (bia_step_noalloc)
 template <bool kDeterministic, bool kRest>
-static void launch_pair_walk(const StepArgs &A, cudaStream_t st)
+static void launch_pair_walk(const StepArgs &A, cudaStream_t st, bool renew = false)
 {
     if (A.nwb <= kWalkBlockMaxPerSm * phase_kernel_setup()) {
+        if (renew) smem_opt_in(bia_pair_walk_block_kernel<kDeterministic, kRest>, walk_block_smem_bytes<kRest>());
         bia_pair_walk_block_kernel<kDeterministic, kRest>
             <<<(unsigned)A.nwb, kWalkBlockWarps * 32, walk_block_smem_bytes<kRest>(), st>>>(A);
         return;
@@ -459,21 +464,24 @@ static void launch_pair_walk(const StepArgs &A, cudaStream_t st)
 }
 
 template <bool kDeterministic>
-static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st, int tuned = -1)
+static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st, int tuned = -1, bool renew = false)
 {
     if (A.P.method == kMethodAlg) {
         const int var = alg_variant_for(A.nwb, tuned);
         if (var == kVarPhase32) {
+            if (renew) smem_opt_in(bia_pair_phase_kernel<kDeterministic, 32, 1>, phase_smem_bytes<32>());
             bia_pair_phase_kernel<kDeterministic, 32, 1>
                 <<<(unsigned)((A.nwb + 31) / 32), 32 * 32, phase_smem_bytes<32>(), st>>>(A);
             return;
         }
         if (var == kVarPhase32Lane) {
+            if (renew) smem_opt_in(bia_pair_phase_kernel<kDeterministic, 32, 1, false>, phase_smem_bytes<32, false>());
             bia_pair_phase_kernel<kDeterministic, 32, 1, false>
                 <<<(unsigned)((A.nwb + 31) / 32), 32 * 32, phase_smem_bytes<32, false>(), st>>>(A);
             return;
         }
         if (var == kVarTiles8 && A.nwb < kBlockMaxPerSm * phase_kernel_setup()) {
+            if (renew) smem_opt_in(bia_pair_block_kernel<kDeterministic>, sizeof(AlgBlockShared));
             bia_pair_block_kernel<kDeterministic>
                 <<<(unsigned)A.nwb, kBlockWarps * 32, sizeof(AlgBlockShared), st>>>(A);
             return;
@@ -482,11 +490,12 @@ static void launch_pair_tiles(const StepArgs &A, long long grid, cudaStream_t st
     switch (A.P.method) {
     case kMethodRkf:
         phase_kernel_setup();
+        if (renew) smem_opt_in(bia_pair_block_rkf_kernel<kDeterministic>, sizeof(RkfBlockShared));
         bia_pair_block_rkf_kernel<kDeterministic>
             <<<(unsigned)(A.nwb < 0x7fffffffLL ? A.nwb : 0x7fffffffLL), kBlockWarps * 32, sizeof(RkfBlockShared), st>>>(A);
         break;
     case kMethodUniversal:
-        launch_pair_walk<kDeterministic, false>(A, st);
+        launch_pair_walk<kDeterministic, false>(A, st, renew);
         break;
     default:
         bia_pair_tiles_kernel<kDeterministic><<<(unsigned)grid, kThreads, 0, st>>>(A);
@@ -1132,6 +1141,8 @@ int bia_context_create(bia_context **out, int device, void *stream)
         bia_context_destroy(ctx);
         return cuda_status(e);
     }
+    g_contexts++;
+    phase_kernel_setup(true);
     *out = ctx;
     return BIA_OK;
 }
@@ -1537,12 +1548,13 @@ static __device__ __align__(256) double g_noalloc_scratch[kNoAllocPartDoubles + 
 // array is only a stand-in: it must be resolved with cudaGetSymbolAddress while the
 // device is current.  It is resolved again on every call made outside stream capture (a
 // cheap query that allocates nothing), so a device reset or a recreated primary context,
-// which loads the module again at a new address, is picked up; during a capture the
-// address of the last call outside capture is used.
+// which loads the module again at a new address, is picked up; the pair kernel's opt-in to
+// its shared memory, which a reset forgets too, is made again with it.  During a capture the
+// address and the opt-in of the last call outside capture are used.
 static double *g_noalloc_addr[kNoAllocMaxDevices] = {};
 static std::mutex g_noalloc_mutex;
 
-static int noalloc_scratch(cudaStream_t s, double **out)
+static int noalloc_scratch(cudaStream_t s, double **out, bool *capturing)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -1551,6 +1563,7 @@ static int noalloc_scratch(cudaStream_t s, double **out)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     e = cudaStreamIsCapturing(s, &cap);
     if (e != cudaSuccess) return cuda_status(e);
+    *capturing = cap != cudaStreamCaptureStatusNone;
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
     if (cap == cudaStreamCaptureStatusNone || !g_noalloc_addr[dev]) {
         void *p = nullptr;
@@ -1572,7 +1585,8 @@ extern "C" int bia_step_noalloc(const bia_config *cfg, int n, double *x, double 
     if (n > kNoAllocMaxN) return set_last_error(BIA_ERR_INVALID_ARGUMENT);  // beyond the fixed scratch
     cudaStream_t s = (cudaStream_t)stream;
     double *part = nullptr;
-    st = noalloc_scratch(s, &part);
+    bool capturing = false;
+    st = noalloc_scratch(s, &part, &capturing);
     if (st != BIA_OK) return set_last_error(st);
     unsigned long long *counters = (unsigned long long *)(part + kNoAllocPartDoubles);
     // the partials are fully rewritten by every step; only the counters start at zero
@@ -1595,7 +1609,7 @@ extern "C" int bia_step_noalloc(const bia_config *cfg, int n, double *x, double 
     A.P.itr = cfg->itr;
     A.P.method = cfg->method;
     const long long grid = (A.nwb + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    launch_pair_tiles<true>(A, grid, s);
+    launch_pair_tiles<true>(A, grid, s, -1, !capturing);
     UpdateArgs U;
     U.x = x; U.y = y; U.z = z; U.u = u; U.v = v; U.w = w;
     U.part = part;
