@@ -314,8 +314,9 @@ static bool smem_opt_in(Kernel *kernel, size_t bytes)
 static std::atomic<unsigned> g_contexts{0};
 
 // Once per device (the current one) and again after a context was created: opt the pair kernels in to their
-// dynamic shared memory and read the SM count.  Returns the SM count, 0 when the set-up failed
-// (the caller then launches the 8-warp kernel).  if_made: only where the set-up was made
+// dynamic shared memory and read the SM count.  Returns the SM count, 0 when the opt-in of a kernel that has another
+// in its place failed (the 8-warp ALG kernel or the walk is then launched); RKF45 has no
+// other kernel, its launch is refused and the step returns the error.  if_made: only where the set-up was made
 // before (a new context makes it again; the first one leaves it, and the kernels' loading, to the first step).
 static int phase_kernel_setup(bool if_made = false)
 {
@@ -330,6 +331,8 @@ static int phase_kernel_setup(bool if_made = false)
     if (if_made && made_of[dev] == 0u) return 0;
     if (made_of[dev] != now) {
         int sms = 0;
+        const bool rkf = smem_opt_in(bia_pair_block_rkf_kernel<true>, sizeof(RkfBlockShared)) &&
+                         smem_opt_in(bia_pair_block_rkf_kernel<false>, sizeof(RkfBlockShared));
         const bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
                         smem_opt_in(bia_pair_phase_kernel<true, 32, 1>, phase_smem_bytes<32>()) &&
                         smem_opt_in(bia_pair_phase_kernel<false, 32, 1>, phase_smem_bytes<32>()) &&
@@ -337,13 +340,11 @@ static int phase_kernel_setup(bool if_made = false)
                         smem_opt_in(bia_pair_phase_kernel<false, 32, 1, false>, phase_smem_bytes<32, false>()) &&
                         smem_opt_in(bia_pair_block_kernel<true>, sizeof(AlgBlockShared)) &&
                         smem_opt_in(bia_pair_block_kernel<false>, sizeof(AlgBlockShared)) &&
-                        smem_opt_in(bia_pair_block_rkf_kernel<true>, sizeof(RkfBlockShared)) &&
-                        smem_opt_in(bia_pair_block_rkf_kernel<false>, sizeof(RkfBlockShared)) &&
                         smem_opt_in(bia_pair_walk_block_kernel<true, false>, walk_block_smem_bytes<false>()) &&
                         smem_opt_in(bia_pair_walk_block_kernel<false, false>, walk_block_smem_bytes<false>()) &&
                         smem_opt_in(bia_pair_walk_block_kernel<true, true>, walk_block_smem_bytes<true>()) &&
                         smem_opt_in(bia_pair_walk_block_kernel<false, true>, walk_block_smem_bytes<true>());
-        if (!ok) cudaGetLastError();  // clear; the 8-warp kernel is used instead
+        if (!ok || !rkf) cudaGetLastError();  // clear
         sms_of[dev] = ok ? sms : 0;
         made_of[dev] = now;
     }
