@@ -192,12 +192,10 @@ struct EnsItems {
 template <bool kRest>
 __global__ void __launch_bounds__(kEnsThreads, 2) ens_pair_walk_kernel(const EnsArgs A)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WalkCounts c = {0, 0, 0, 0};
+    const int warp = threadIdx.x >> 5;
     uv_walk_blocks<true, kRest>(EnsItems{A}, (long long)blockIdx.x * kEnsWarps + warp,
                                 (long long)gridDim.x * kEnsWarps, A.nitems, A.P.dt, warp * walk_warp_doubles<kRest>(),
-                                A.R, c);
-    walk_flush_counts(c, A.stats, lane);
+                                A.R, A.stats);
 }
 
 // Learned step over the item table, third kernel (persistent 8-warp CTAs): a dense or

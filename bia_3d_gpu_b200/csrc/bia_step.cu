@@ -421,17 +421,15 @@ struct StepItems {
 // (kRest true: a pair that is not exact by series and inside a head's domain is deferred, its head
 // input to the rows, its block to the list): a persistent grid of kPersistentCtas CTAs per SM
 // (128 registers a thread; three or four CTAs with the registers that leaves are slower, 4.36 to 4.62
-// against 4.10 ms a step on plummer_32768), the counters flushed once per warp.  Deterministic
+// against 4.10 ms a step on plummer_32768), the counters flushed per warp.  Deterministic
 // mode writes every partial slot here.
 template <bool kDeterministic, bool kRest>
 __global__ void __launch_bounds__(kThreads, kPersistentCtas) bia_pair_walk_kernel(const StepArgs A)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WalkCounts c = {0, 0, 0, 0};
+    const int warp = threadIdx.x >> 5;
     uv_walk_blocks<kDeterministic, kRest>(StepItems{A}, (long long)blockIdx.x * kWarpsPerBlock + warp,
                                           (long long)gridDim.x * kWarpsPerBlock, A.nwb, A.P.dt,
-                                          warp * walk_warp_doubles<kRest>(), A.R, c);
-    walk_flush_counts(c, A.stats, lane);
+                                          warp * walk_warp_doubles<kRest>(), A.R, A.stats);
 }
 
 // The same by a CTA per warp-block (uv_block_solve), up to kWalkBlockMaxPerSm warp-blocks per SM, one wave of

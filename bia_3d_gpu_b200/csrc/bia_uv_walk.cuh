@@ -202,6 +202,23 @@ struct WalkCounts {
     int pairs, iters, over, nonfinite;  // universal-variable pairs, Newton iterations, not converged
 };
 
+// The warp's counts onto the context's counters.
+__device__ __forceinline__ void walk_flush_counts(const WalkCounts &c, unsigned long long *stats, int lane)
+{
+    PairCounters p;
+    counters_zero(p);
+    p.cls[kUniversal] = c.pairs;
+    p.it_uv = c.iters;
+    p.nonconverged = c.over;
+    p.nonfinite = c.nonfinite;
+    flush_counters(p, stats, lane);
+}
+
+// A walk flushes its counts every this many blocks: 1024 pairs each, of at most kUvItMax + 1 iterations, stay
+// below 2^31 summed over a warp.
+constexpr int kWalkFlushBlocks = 8192;
+static_assert(1024LL * (kUvItMax + 1) * kWalkFlushBlocks < 1LL << 31, "");
+
 // One pair of the second kind: its displacement in h (uv: returns kLearnedPlain always), or its head and
 // head input x01.  Counted in c unless deferred.
 template <bool kRest>
@@ -535,18 +552,20 @@ __device__ __forceinline__ void uv_block_solve(const Items &I, long long t, doub
 
 // The walk of a persistent grid: warp `first` of `stride` warps takes blocks first, first + stride, ... of
 // `count`.  I.block(t) gives block t, I.system(s) a system; `slice` is where the warp's doubles
-// (walk_warp_doubles) begin in the dynamic shared memory.
+// (walk_warp_doubles) begin in the dynamic shared memory.  The counts go to stats.
 template <bool kDeterministic, bool kRest, class Items>
 __device__ __forceinline__ void uv_walk_blocks(const Items &I, long long first, long long stride, long long count,
-                                               double dt, int slice, const LearnedRows &R, WalkCounts &c)
+                                               double dt, int slice, const LearnedRows &R, unsigned long long *stats)
 {
     const int lane = threadIdx.x & 31;
+    WalkCounts c = {0, 0, 0, 0};
     double *ws = warp_slices + slice;
     WalkBlock *blocks = reinterpret_cast<WalkBlock *>(ws + kTileSmemDoubles);
     unsigned int *queue = reinterpret_cast<unsigned int *>(blocks + kQueuePairs);
     uint32_t *wslots = reinterpret_cast<uint32_t *>(ws + kWalkSliceDoubles);
     const UvFastStep T = uv_fast_step(dt);
     int qn = 0, nblocks = 0;  // pairs and blocks in the queue
+    int uncounted = 0;        // blocks since the counts were flushed
     for (long long t = first;; t += stride) {  // warp-uniform
         const bool have = t < count;
         unsigned left = 0u, others = 0u;
@@ -590,25 +609,18 @@ __device__ __forceinline__ void uv_walk_blocks(const Items &I, long long first, 
             walk_queue<kDeterministic, kRest>(I, R, dt, queue, blocks, qn, lane, c);
             qn = nblocks = 0;
         }
-        if (!have) return;
+        if (!have || ++uncounted == kWalkFlushBlocks) {
+            walk_flush_counts(c, stats, lane);
+            if (!have) return;
+            c = {0, 0, 0, 0};
+            uncounted = 0;
+        }
         if (others != 0u) {
             walk_queue_push(queue, blocks, B, left, qn, nblocks, lane);
             nblocks++;
             qn += (int)others;
         }
     }
-}
-
-// The warp's counts onto the context's counters.
-__device__ __forceinline__ void walk_flush_counts(const WalkCounts &c, unsigned long long *stats, int lane)
-{
-    PairCounters p;
-    counters_zero(p);
-    p.cls[kUniversal] = c.pairs;
-    p.it_uv = c.iters;
-    p.nonconverged = c.over;
-    p.nonfinite = c.nonfinite;
-    flush_counters(p, stats, lane);
 }
 
 }  // namespace bia
