@@ -1045,7 +1045,8 @@ __device__ __forceinline__ void uv_compose_series(const UvPair &p, const UvSerie
 // (F(0) = -dt < 0; hi < 0 until an upper bound is seen).  A Newton step that leaves the
 // bracket, or is not below half the step before last, is replaced by bisection, so the
 // bracket at least halves every two iterations: on hyperbolic branches Newton from far
-// above the root moves only ~1/sqrt(-beta) per step.  Returns the iterations
+// above the root moves only ~1/sqrt(-beta) per step.  So is a step where 1/F' is not a normal
+// number (rcp_normal: 0, which would look converged).  Returns the iterations
 // (kUvItMax + 1 when the cap was reached).
 // ifp (optional): 1 / F' at the last evaluation, for uv_compose (F' = r(s)).
 __device__ __forceinline__ int uv_iterate(const UvPair &p, double dt, double &s_io, double *ifp = nullptr)
@@ -1062,13 +1063,14 @@ __device__ __forceinline__ int uv_iterate(const UvPair &p, double dt, double &s_
         if (F == 0.0) break;
         ifp_last = rcp_normal(Fp);
         const double step = F * ifp_last;
-        if (Fp > 0.0 && fabs(step) <= 4.0 * 2.220446049250313e-16 * fabs(s)) {
+        const bool slope = Fp > 0x1p-1021 && Fp < 0x1p1021;
+        if (slope && fabs(step) <= 4.0 * 2.220446049250313e-16 * fabs(s)) {
             s = s - step;  // converged: the remaining correction is a few ulps
             break;
         }
         if (F < 0.0) lo = s; else hi = s;  // a NaN F (overflow far above the root) lowers hi
         double sn = s - step;
-        const bool newton = (Fp > 0.0) && (sn > lo) && (hi < 0.0 || sn < hi) &&
+        const bool newton = slope && (sn > lo) && (hi < 0.0 || sn < hi) &&
                             (hi < 0.0 || fabs(step) <= 0.5 * dxold);
         if (!newton) sn = (hi > 0.0) ? 0.5 * (lo + hi) : 2.0 * s;
         dxold = dx;
@@ -1085,7 +1087,8 @@ __device__ __forceinline__ int uv_iterate(const UvPair &p, double dt, double &s_
 }
 
 // One Halley step on the same equation from s: returns the step ds (s_new = s - ds).
-// F'' = dr/ds = sig c0 + (mu - beta r0) s c1.
+// F'' = dr/ds = sig c0 + (mu - beta r0) s c1.  NaN where the reciprocal is not a normal number (rcp_normal: 0,
+// which would look converged): learned_finish leaves the pair to uv_iterate.
 __device__ __forceinline__ double uv_halley_step(const UvPair &p, double dt, double s)
 {
     double c[4];
@@ -1093,7 +1096,8 @@ __device__ __forceinline__ double uv_halley_step(const UvPair &p, double dt, dou
     const double F = p.r0 * s * c[1] + p.sig * s * s * c[2] + p.mu * s * s * s * c[3] - dt;
     const double Fp = p.r0 * c[0] + p.sig * s * c[1] + p.mu * s * s * c[2];
     const double Fpp = p.sig * c[0] + (p.mu - p.beta * p.r0) * s * c[1];
-    return F * Fp * rcp_normal(Fp * Fp - 0.5 * F * Fpp);
+    const double den = Fp * Fp - 0.5 * F * Fpp;
+    return den < 0x1p1021 ? F * Fp * rcp_normal(den) : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 // Half-displacement from the solved s: f - 1, g - dt, f', g' - 1 from the Stumpff
