@@ -71,6 +71,10 @@ __device__ __forceinline__ double rsqrt_normal(double x)
     return fma(fma(e, 0.375, 0.5), __dmul_rn(y, e), y);
 }
 
+// The same of any x.
+static __device__ __noinline__ double rsqrt_small(double x) { return rsqrt(x); }
+__device__ __forceinline__ double rsqrt_any(double x) { return x > 1e-290 ? rsqrt_normal(x) : rsqrt_small(x); }
+
 // c x^(-3/2) of a normal x from the same approximation y, whose square is exact (its low half is zero):
 // c y^3 (1 + 3/2 e + 15/8 e^2), e = 1 - x y^2; the next term, 35/16 e^3, is below 3e-17.
 __device__ __forceinline__ double scaled_rsqrt3_normal(double c, double x)
@@ -132,8 +136,8 @@ __device__ __forceinline__ bool frame_xi_eta(const double r[3], const double g[3
         return true;
     }
     double ez[3];
-    const double iL = Lsq > 1e-290 ? rsqrt_normal(Lsq) : 1.0 / sqrt(Lsq);
-    const double ig = gsq > 1e-290 ? rsqrt_normal(gsq) : 1.0 / gm;
+    const double iL = rsqrt_any(Lsq);
+    const double ig = rsqrt_any(gsq);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         e_eta[k] = g[k] * ig;
@@ -244,6 +248,9 @@ static __device__ __noinline__ double hyp_guess(const HypConsts c, double *error
 // not small against the distance to the asymptotes (below 1e-3 of it the step's error is 1e-6, and the
 // guess, an angle from scratch, never the better one).
 //
+// The squares of distance, velocity and angular momentum have to be normal numbers (rsqrt_normal): below about
+// 1e-154 of each a pair comes out non-finite and is counted so.  Nothing else leaves the type's range before they do.
+//
 // What bounds the ALG kernels: FP64 operations in dependent chains (atan2, log, and a sine, cosine and log an
 // evaluation), 46 % of the FP64 pipe and 68 % of the issue slots at 22 of 32 lanes on mixed classes.  So the
 // work per pair is what counts.  Step at n = 32768, Plummer / Coulomb: 71.0 / 83.0 ms with divisions, roots and
@@ -267,14 +274,14 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
     const double ig_0 = rsqrt_normal(W);
     const double g_0 = W * ig_0;
     const double bg = eps_th * ig_0;           // b_0 g_0
-    const double b_g = bg * (ig_0 * ig_0);     // b_0 / g_0
-    const double g_b = g_0 * W * rcp_normal(eps_th);  // g_0 / b_0
+    const double b_g = (bg * ig_0) * ig_0;     // b_0 / g_0, without the cube of a velocity
     const double b = aL * ig_0;
     HypConsts c;
     const double iden0 = rsqrt_normal(bg * bg + Lz * Lz);
     c.cs_0 = bg * iden0;
     c.sn_0 = aL * iden0;
-    c.tn_0 = aL * (g_0 * rcp_normal(eps_th));
+    const double ieps = rcp_normal(eps_th);
+    c.tn_0 = aL * (g_0 * ieps);
     half_angle(c.sn_0, c.cs_0, c.s0h, c.c0h);
     // the start: sine, cosine and angle
     const double bs = b * c.sn_0;
@@ -302,7 +309,7 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
     const double tau_ini = c.tn_0 * sn * Dinv_i + (sn >= 0.0 ? -lq : lq);
     const double time_ini = tau_ini * b_g;
     const double time_end = time_ini + sgn * dt;
-    c.time_end_ = time_end * g_b;
+    c.time_end_ = (time_end * g_0) * (W * ieps);  // time_end g_0 / b_0
 
     // the start of the iteration: one Newton step on (its residual is known already), or the guess
     const double error_ini_ = tau_ini - c.time_end_;
@@ -313,8 +320,9 @@ __device__ __forceinline__ int hyperbola(double eps_th, double dt, int ITR, cons
     if (fabs(step_ini) <= 1e-3 * (big * q_i)) {  // big q_i: the sine of half the smaller distance
         // on from the Newton step by theta(t)'s Taylor series to third order (theta' = L/r^2,
         // r'' = L^2/r^3 + eps/r^2): the first evaluation then meets the rounding floor
-        const double rho = r_g * (ir * ir) * dt;
-        const double kap = (Lz * Lz * ir + eps_th) * (ir * ir * ir) * (dt * dt);
+        const double tr = ir * dt;
+        const double rho = (r_g * ir) * tr;
+        const double kap = ((Lz * Lz * ir + eps_th) * ir) * (tr * tr);
         theta_end = theta_ini - step_ini * (1.0 + (rho * rho - rho - kap * (1.0 / 3.0)));
     } else {
         double error_gss_;
@@ -538,8 +546,8 @@ static __device__ __noinline__ int ellipse(double eps_th, double dt, int ITR, co
     const double uu_end = -gr * sn_end;
     const double vv_end = b * ia * gr * cs_end;
     // the rotation from the orbit's frame: the start's position in both (the reference takes the
-    // difference of the two angles by atan2, and its sine and cosine back)
-    const double in = rsqrt_normal((px * px + py * py) * r2);
+    // difference of the two angles by atan2, and its sine and cosine back); no fourth power of a distance
+    const double in = rsqrt_normal(px * px + py * py) * ir;
     const double cs_alp = (px * X_ini + py * Y_ini) * in, sn_alp = (px * Y_ini - py * X_ini) * in;
     YN[0] = xx_end * cs_alp - yy_end * sn_alp;
     YN[1] = xx_end * sn_alp + yy_end * cs_alp;
