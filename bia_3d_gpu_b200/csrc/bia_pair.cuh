@@ -1105,7 +1105,7 @@ __device__ __forceinline__ double uv_halley_step(const UvPair &p, double dt, dou
     const double Fp = p.r0 * c[0] + p.sig * s * c[1] + p.mu * s * s * c[2];
     const double Fpp = p.sig * c[0] + (p.mu - p.beta * p.r0) * s * c[1];
     const double den = Fp * Fp - 0.5 * F * Fpp;
-    return den < 0x1p1021 ? F * Fp * rcp_normal(den) : __longlong_as_double(0x7ff8000000000000LL);
+    return den < 0x1p1021 ? F * (Fp * rcp_normal(den)) : __longlong_as_double(0x7ff8000000000000LL);
 }
 
 // Half-displacement from the solved s: f - 1, g - dt, f', g' - 1 from the Stumpff

@@ -10,12 +10,13 @@ after five to six duplications, each of which can multiply a relative rounding e
 4.5e-13, twice (the root's error and the composition's), and a little for the sums: 2e-12.
 
 The learned pair's Halley step where F'^2 is there, separations of 2^511, among smaller and unscaled ones: what
-it accepts is off by 1e-15 at most, the composition as above."""
+it accepts is off by 1e-15 at most, the composition as above.  And where the residual times F' is infinite
+(lengths of 2^480, velocities of 2^-300): an infinite step is no accepted one."""
 import numpy as np
 import pytest
 
 import oracle
-from bia_3d_gpu_b200 import METHOD_LEARNED, METHOD_UNIVERSAL, BIASolver, default_config
+from bia_3d_gpu_b200 import METHOD_LEARNED, METHOD_UNIVERSAL, BIASolver, default_config, initial
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +64,21 @@ def test_learned_pair_of_extreme_size(cuda, scale, v):
     for part in (slice(0, 3), slice(3, 6)):
         unit = r0 if part.start == 0 else v0
         assert np.linalg.norm(got[part, 0] / unit - want[part] / unit) <= 2e-12 * np.linalg.norm(want[part] / unit)
+
+
+@pytest.mark.parametrize("eps", [-0.05, -20.0])
+def test_learned_residual_beyond_the_range(cuda, eps):
+    s, _ = initial.plummer(6, seed=9)
+    sums = []
+    with BIASolver() as solver:
+        solver.load_heads()
+        for a, b in ((0, 0), (480, -300)):
+            unit = 2.0 ** np.array([a, a, a, b, b, b])[:, None]
+            t = cuda.tensor(s * unit, device="cuda")
+            out = cuda.zeros_like(t)
+            cfg = default_config(eps_th=float(np.ldexp(eps, a + 2 * b)), dt=float(np.ldexp(2e-2, a - b)), method=METHOD_LEARNED)
+            st = solver.step_shard(t, cfg, 0, 1, out, stats=True)
+            assert st["nonfinite"] == 0 and st["learned"] > 0
+            sums.append(out.cpu().numpy() / unit)
+    for part in (slice(0, 3), slice(3, 6)):
+        assert np.abs(sums[1][part] - sums[0][part]).max() <= 2e-12 * np.abs(sums[0][part]).max()
