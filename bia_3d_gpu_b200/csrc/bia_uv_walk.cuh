@@ -361,6 +361,23 @@ __device__ __forceinline__ void walk_queue(const Items &I, const LearnedRows &R,
     __syncwarp();
 }
 
+// Whether the short step may take a block's pairs: eps_ij dt^2 of every coupling that is not zero has to be a normal
+// number (below, uv_fast_pair would lose bits of the interaction or all of it; an infinite one gives NaN, which it
+// refuses), and so have its factors in that order.  cdt2: eps dt^2 times the lane's row charge qi; qj: the charge of
+// its column.  The same on every lane.
+__device__ __forceinline__ bool walk_coupling_normal(const WalkSystem &S, double dt2, double cdt2, double qi, double qj)
+{
+    constexpr int kOne = 1023 << 20, kLeast = (1023 - 960) << 20;  // 1 and 2^-960 as high words
+    if (S.eps_th == 0.0) return true;
+    const int e = __double2hiint(fabs(S.eps_th * dt2));
+    if (!S.q || e < kLeast) return e >= kLeast;
+    int a = qi != 0.0 ? __double2hiint(fabs(cdt2)) : kOne;
+    int b = qj != 0.0 ? __double2hiint(fabs(qj)) : kOne;
+    a = __reduce_min_sync(0xffffffffu, a);
+    b = __reduce_min_sync(0xffffffffu, b);
+    return a >= kLeast && a >= kLeast + (kOne - b);  // the high words of a product add up, but for kOne
+}
+
 // What a block's sums lack after its first pass: the half-displacement's constant factors, and
 // velocities over dt (uv_fast_pair).
 __device__ __forceinline__ void walk_scale(const UvFastStep &T, double *ws, int lane, double racc[6])
@@ -476,6 +493,7 @@ __device__ __forceinline__ void uv_block_solve(const Items &I, long long t, doub
     const bool full_block = !diag && ncols >= 32;
     const int k0 = diag ? 1 : 0, k1 = diag ? 16 : 31;
     UvRow row;
+    bool fast = T.on;  // the same for the CTA
     {
         double si[7];
         load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, i, si);
@@ -485,17 +503,18 @@ __device__ __forceinline__ void uv_block_solve(const Items &I, long long t, doub
             row.s[d] = si[d];
             row.s[3 + d] = si[3 + d] * T.dt;
         }
-    }
-    if (warp == 0) {
-        double sj[7];
-        load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, B.bj * 32 + lane, sj);
+        if (warp == 0) {
+            double sj[7];
+            load_particle(S.x, S.y, S.z, S.u, S.v, S.w, S.q, S.n, B.bj * 32 + lane, sj);
+            fast = fast && walk_coupling_normal(S, T.dt2, row.cdt2, si[6], sj[6]);
 #pragma unroll
-        for (int d = 3; d < 6; d++) sj[d] *= T.dt;
-        slice_fill(ws, lane, sj);
-        lefts[lane] = 0u;
+            for (int d = 3; d < 6; d++) sj[d] *= T.dt;
+            slice_fill(ws, lane, sj);
+            lefts[lane] = 0u;
+        }
     }
-    __syncthreads();
-    if (T.on) {  // the same for the CTA
+    fast = __syncthreads_and(fast);
+    if (fast) {
         unsigned mine = 0u;
         for (int k = k0 + warp; k <= k1; k += kWalkBlockWarps) {
             const int src = (lane + k) & 31;
@@ -531,7 +550,7 @@ __device__ __forceinline__ void uv_block_solve(const Items &I, long long t, doub
     if (warp != 0) return;
     unsigned left;
     double racc[6];
-    if (T.on) {
+    if (fast) {
         left = lefts[lane];
         if (full_block && __reduce_add_sync(0xffffffffu, (unsigned)__popc(left & ((1u << kProbe) - 1u))) > 32u * kProbe / 4u)
             left |= 0xffffffffu << kProbe;
@@ -591,7 +610,7 @@ __device__ __forceinline__ void uv_walk_blocks(const Items &I, long long first, 
                 }
                 slice_fill(ws, lane, sj);
                 __syncwarp();
-                if (T.on) {
+                if (T.on && walk_coupling_normal(S, T.dt2, row.cdt2, si[6], sj[6])) {
                     if (!diag && ncols >= 32) {
                         left = S.q ? uv_walk_full<true>(slice, row, lane, racc) : uv_walk_full<false>(slice, row, lane, racc);
                     } else {
