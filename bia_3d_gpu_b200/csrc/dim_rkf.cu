@@ -374,7 +374,7 @@ struct DimCoopArgs {
 // component); thread (particle lane, chunk c) of the block's P x C threads (C = 256 / P)
 // adds the tile's entries c, c + C, ..., and the C chunk sums of a particle are added in
 // chunk order at the end (deterministic).  P = 32: each tile serves 32 particles, 32 entries per
-// thread.  It takes the sizes beyond the resident kernel below (about 35000 particles on 148 SMs).
+// thread.  It takes the sizes beyond the resident kernel below (more than 224 particles a CTA, 33152 on 148 SMs).
 //
 // Inverse cube: kFastInv (bia_dim_integrate) eps r^-3 from one rsqrt (r^-1, then its cube;
 // rsqrt is within 1 ulp, the product within ~4 ulp of eps / r^3); otherwise the
@@ -1155,7 +1155,7 @@ static int dim_integrate_coop(DimRun &R, double *y, double *x0, double xe, int i
         B.io = R.B.io;
         args[0] = (void *)&B;
     } else {
-        // too many particles for the SMs' shared memory: groups of 32, all state in global memory
+        // too many particles for a CTA per SM (dim_resident_plan): groups of 32, all state in global memory
         kern = R.fast_inv ? (const void *)dim_coop_kernel<32, true> : (const void *)dim_coop_kernel<32, false>;
         bytes = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1) {
