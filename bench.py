@@ -83,8 +83,8 @@ METHODS = {"rkf": 0, "alg": 1, "universal": 2, "learned": 3}
 # The learned step's dominant kernel is the rest pass's walk (it writes every partial slot; the head
 # and finish kernels move under 1 MB at this size on this workload).
 TRAFFIC = {
-    ("plummer_32768", 3, "split"): (16384 * 16383 // 2, 66.538e6 + 418.112e6),
-    ("coulomb_cube_32768", 1, None): (16384 * 16383 // 2, 9.913e6 + 1528.214e6),  # phase-locked ALG
+    ("plummer_32768", 3, "split"): (16384 * 16383 // 2, 68.834e6 + 418.967e6),
+    ("coulomb_cube_32768", 1, None): (16384 * 16383 // 2, 8.627e6 + 1754.595e6),  # phase-locked ALG
 }
 
 
@@ -263,6 +263,14 @@ def metric_name(method):
     if method == "learned":
         return "BIA pair-updates/s: learned-guess form vs plain FP64, at <=1e-12 pos. error"
     return "BIA pair-updates/s (plain FP64 step)"
+
+
+def precision_note(method):
+    """What a method computes in what precision (RKF45 and ALG: FP64)."""
+    short = "FP64; short-step pairs' series terms from the third order on (below 1e-10 of a pair's displacement) FP32"
+    if method == 3:
+        return "heads: BF16 operands, FP32 accumulation; first correction FP32; final step, composition and sums " + short
+    return short if method == 2 else "FP64"
 
 
 def _init_dist(world):
@@ -774,9 +782,7 @@ def main():
             "scaling": "strong" if shard else "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded)",
             "config": config_keys(args.workload, n, dt, args.method, world, reduction="deterministic",
-                                  precision=("heads: BF16 operands, FP32 accumulation; first correction "
-                                             "FP32; final step, composition and sums FP64"
-                                             if method == 3 else "FP64"),
+                                  precision=precision_note(method),
                                   l2="256 MB buffer written between timed steps (untimed)",
                                   state="reset to the seeded state before every timed step (untimed "
                                         "device copy; the e2e loop runs consecutive steps from it through host buffers)",

@@ -75,8 +75,9 @@ __device__ __forceinline__ double rsqrt_normal(double x)
 static __device__ __noinline__ double rsqrt_small(double x) { return rsqrt(x); }
 __device__ __forceinline__ double rsqrt_any(double x) { return x > 1e-290 ? rsqrt_normal(x) : rsqrt_small(x); }
 
-// c x^(-3/2) of a normal x from the same approximation y, whose square is exact (its low half is zero):
-// c y^3 (1 + 3/2 e + 15/8 e^2), e = 1 - x y^2; the next term, 35/16 e^3, is below 3e-17.
+// c x^(-3/2) of a normal x from the same approximation y, whose square is exact (its low half is zero), and one step
+// of Householder's third-order iteration: c y^3 (1 + 3/2 e + 15/8 e^2), e = 1 - x y^2; the next term, 35/16 e^3,
+// is below 3e-17.
 __device__ __forceinline__ double scaled_rsqrt3_normal(double c, double x)
 {
     double y;
@@ -87,8 +88,9 @@ __device__ __forceinline__ double scaled_rsqrt3_normal(double c, double x)
     return fma(c3 * e, fma(e, 1.875, 1.5), c3);
 }
 
-// 1/x of a normal x with a normal reciprocal: the hardware approximation y and one third-order step
-// y (1 + e + e^2), e = 1 - x y (the next term, e^3, is below 1e-17).  Zero gives NaN.
+// 1/x of a normal x with a normal reciprocal: the hardware approximation y and one step of Householder's
+// third-order iteration, y (1 + e + e^2), e = 1 - x y (the next term, e^3, is below 1e-17).  Zero gives NaN; 2^1022
+// and beyond, whose reciprocals are subnormal, give 0, which a Newton step must not take for a root (uv_iterate).
 __device__ __forceinline__ double rcp_normal(double x)
 {
     double y;
@@ -668,7 +670,8 @@ __device__ __forceinline__ void moon_acc(double eps_th, double x, double y, doub
 // a1 = (ax, ay); er written when kWantEr.  A position's derivative is the stage's velocity
 // u0 + h sum_m B_sm a_m, so the position of stage s is x0 + c_s h u0 + h^2 sum_m N_sm a_m with
 // N = B B (and GA B, DA B for the new position and its error): the accelerations are all that is
-// kept, no stage velocity is formed, and a step takes 62 operations for its sums instead of 100.
+// kept, no stage velocity is formed, and a step takes 62 operations for its sums instead of 100.  (h^2 has to be a
+// normal number: below |h| of 1e-154 the accelerations do not reach the positions.)
 struct FehlbergNested {
     using F = Fehlberg;
     static constexpr double N31 = F::B32 * F::B21;
@@ -1203,7 +1206,8 @@ __device__ __forceinline__ int uv_halfdisp_fast(double eps_th, double dt, const 
 // formed in FP32: their rounding stays below 2e-17 of the result.  What is left out (p5 beyond -a p4,
 // g4 in g - dt, the sixth order) is below that too.  Everything from p2 down is FP64.
 //
-// It works on w (velocities times dt, so that neither dt/r0 nor its square is formed) and leaves the
+// It works on w (relative velocities times dt, so that neither dt/r0 nor its square is formed; the difference is taken
+// before the product, walk_diff) and leaves the
 // constant factors of the half-displacement to the sums: h = 1/4 (H[0..2]) and (1/2)/dt (H[3..5]).
 // Returns false, H undefined, for any other pair: the caller takes the general solver.  Every
 // operation is written out, so that each kernel that inlines it computes the same bits; H

@@ -1,15 +1,14 @@
 // bia_step.cu -- the BIA pair step on B200: tile kernel, reduction, context and API.
 //
 // Work decomposition.  The pairs i<j form the upper triangle of an n x n matrix.  It
-// is cut into 32 x 32 warp-blocks (bi <= bj, 32-particle row and column blocks); one
-// warp owns one warp-block.  Lane l keeps its row particle i = 32*bi + l and its
-// column particle j = 32*bj + l in registers.  At rotation step k lane l pairs its
-// row with column slot (l + k) mod 32, fetched from that lane with a shuffle, so
-// every lane solves a different pair and the column slot's accumulator can be
-// handed back by a second shuffle from lane (l - k) mod 32.  Off-diagonal blocks take
-// 32 rotation steps (1024 pairs), diagonal blocks 16 (k = 1..15 on all lanes, k = 16
-// on lanes 0..15: the 496 pairs of the block once each; orientation does not matter
-// because the half-displacement is exactly antisymmetric under i <-> j).
+// is cut into 32 x 32 warp-blocks (bi <= bj, 32-particle row and column blocks); a warp, or
+// for small systems and RKF45 a CTA, owns one.  Lane l has row particle i = 32*bi + l; the
+// column particles and their sums lie in shared memory.  At rotation offset k lane l pairs its
+// row with column slot (l + k) mod 32, so every lane solves a different pair and adds to a
+// different column.  Off-diagonal blocks have 32 offsets (1024 pairs), diagonal blocks 16
+// (k = 1..15 on all lanes, k = 16 on lanes 0..15: the 496 pairs of the block once each;
+// orientation does not matter because the half-displacement is exactly antisymmetric under
+// i <-> j).
 //
 // Reduction.  Each warp-block leaves 32 row sums and 32 column sums of the six
 // half-displacement components.  Deterministic mode writes them to a partial buffer
@@ -179,7 +178,7 @@ __device__ __forceinline__ void block_write(const StepArgs &A, int bi, int bj, i
 // most of the chip idle and a step lasts as long as one warp's 32 turns of a solver.  What is left is
 // a CTA's chain (four turns, the sums) when there are few blocks, else the FP64 pipes.  Three CTAs
 // of 8 warps per SM (85 registers; their 62 KB of h and states leave L1 enough for the spills) let
-// one's sums overlap another's solves: gravity ball of 1332, 82 us a step against 88 with two CTAs
+// one's sums overlap another's solves: gravity ball of 1332, 82 us a graph-replayed step against 88 with two CTAs
 // (128 registers, no spills), 94 and 111 with 16-warp CTAs, two and one per SM, and 137 with
 // bia_pair_tiles_kernel; of 257, 34 against 32, 31, 28 and 137; Coulomb cube of 1332, 123 against
 // 132, 141, 185 and 219.
@@ -277,8 +276,8 @@ __global__ void __launch_bounds__(kBlockWarps * 32, 2) bia_pair_block_rkf_kernel
 //                 registers: all-hyperbolic systems, where packing saves no turn)
 //   kVarPhase32   phase-locked CTAs of 32 warps, 1 per SM (64 registers), balanced class
 //                 loops (mixed classes)
-// All shapes give bitwise the same step.  Measured, us a step (gravity ball, hyperbolic | Coulomb
-// cube, mixed):
+// All shapes give bitwise the same step.  Measured, us a step launched from the host, its two launches and the
+// reduction in it, more than a graph's (gravity ball, hyperbolic | Coulomb cube, mixed):
 //   n       warp-blocks/SM   block          tiles          phase32
 //   1332        6.1           99 |  137     144 |  223     300 |  387
 //   2000       13.6          169 |  281     184 |  301     300 |  391

@@ -11,9 +11,9 @@
 // against 3.80 ms for the learned step of the 32768-body Plummer sphere, 8.7 against 6.2 ms for that of
 // 4096 small ones.  With every pair taking uv_series and its composition in the walk: 5.70 and 8.87 ms.
 //
-// What bounds the walk: the register file's read ports and the FP64 pipe.  A pair takes about 74
+// What bounds the walk: the register file's read ports and the FP64 pipe.  A pair takes about 77
 // FP64 instructions (2 cycles each, 3 where a multiply-add reads three registers) and 75 others; at
-// n = 16384 the FP64 pipe is 58 % and the issue slots 62 % busy, 260 cycles per 32 pairs and scheduler.
+// n = 16384 the FP64 pipe is 60 % and the issue slots 62 % busy, 263 cycles per 32 pairs and scheduler.
 #pragma once
 #include "bia_learned_block.cuh"
 #include "bia_pair.cuh"
